@@ -531,6 +531,9 @@ static int setup_instance(amcfd_ctx *ctx, Inst<T> &I)
     set_sweep_smem_limit<T>(I.line_smem);
     setup_box_solve<T>(I, !ctx->serial_launch);
     if (ctx->box_ctas > 0 && I.box_grid > 0) I.box_grid = std::min(ctx->box_ctas, I.box_grid);
+    // the one-launch chain, unless the caller pins another momentum path
+    setup_mom_chain<T>(I, !ctx->serial_launch && ctx->small_mode == 0 && ctx->box_ctas == 0);
+    if (I.chain_nc > 0 && (rc = alloc3<double>(ctx, &I.rcell, (size_t)5 * I.rcap))) return rc;
     if (sizeof(T) == 4 && I.box_grid > 0)  // the FP32 box solve's tagged exchange of line values
         if ((rc = alloc3<unsigned long long>(ctx, &I.xchg, n3))) return rc;
     I.sweep_warps_max = set_rounds_smem_limit<T>(p);
@@ -657,12 +660,20 @@ static void swap_props(Inst<T> &I)
 template <typename T>
 static bool small_allowed(const amcfd_ctx *ctx, const Inst<T> &I)
 {
+    if (I.chain_nc > 0) return true;
     if (ctx->order != AMCFD_ORDER_REDBLACK || ctx->small_mode == 1) return false;
     return ctx->small_mode == -1 || I.box_grid == 0;
 }
 template <typename T>
 static bool mom_small(const amcfd_ctx *ctx, const Inst<T> &I)
 {
+    if (I.chain_nc > 0) {
+        const Status *s = ctx->st_host;
+        return ctx->last_box >= 0 &&
+               (!s->momentum_active || chain_box_fits(s->iendm1 - s->istatp1 + 1, s->jend - s->jstat + 1,
+                                                      I.p.nkm2 - s->kstat + 1, ctx->order == AMCFD_ORDER_EXACT,
+                                                      I.chain_nc));
+    }
     return small_allowed(ctx, I) && ctx->last_box >= 0 && ctx->last_box <= mom_small_capacity<T>(I);
 }
 
@@ -787,7 +798,7 @@ static int begin_step(amcfd_ctx *ctx)
     h->jstart = ctx->jstart;
     h->lp_niter = 0;
     h->lp_box = ctx->last_box;
-    h->lp_mode = 0;
+    h->lp_mode = ctx->precision == AMCFD_PREC_FP64 ? mom_small<double>(ctx, ctx->I64) : mom_small<float>(ctx, ctx->I32);
     h->lp_small = 0;
     // the per-step block is the leading members of Status, up to heat_iter
     CK(cudaMemcpyAsync(ctx->st_dev, h, offsetof(Status, heat_iter), cudaMemcpyHostToDevice,
@@ -851,6 +862,8 @@ static long long phase_launches(const amcfd_ctx *ctx, int phase, bool small)
         // applyBCs, assembly, factorisation and sweeps, then correctPressure
         const bool coop = (ctx->precision == AMCFD_PREC_FP64 ? ctx->I64.box_grid : ctx->I32.box_grid) > 0;
         const int tickets = ctx->order == AMCFD_ORDER_EXACT ? 1 : 0;
+        const int chain = ctx->precision == AMCFD_PREC_FP64 ? ctx->I64.chain_nc : ctx->I32.chain_nc;
+        if (small && chain > 0) return 1;
         if (small) return ctx->mom_cluster > 1 ? 14 : 9;
         return coop ? 2 + 4 * 2 : tickets + 1 + 4 * (3 + sweeps) + 2 + 1;
     }
@@ -1009,7 +1022,7 @@ static int build_loop_graph(amcfd_ctx *ctx, Inst<T> &I, cudaGraphExec_t &ge)
         swap_props<T>(I);
     }
     cudaGraph_t g_init = capture([&] {
-        const LoopCtl lc{0, hm[1], 1, 1, maxit, cap};
+        const LoopCtl lc{0, hm[1], 1, 1, maxit, cap, I.chain_nc, ctx->order == AMCFD_ORDER_EXACT};
         launch_loop_init(ctx->st_dev, lc, I.stream);
     });
     // top: init, iteration 1, then iterations 2..maxit in sequence, each inside an
@@ -1034,7 +1047,8 @@ static int build_loop_graph(amcfd_ctx *ctx, Inst<T> &I, cudaGraphExec_t &ge)
         if (cap >= 0) child(br[0], nullptr, mom_small_g[q]);
         child(br[1], nullptr, mom_grid_g[q]);
         // species and the convergence test, with the loop control of iteration k
-        const LoopCtl lc{k < maxit ? hc[k] : 0, k < maxit ? hm[k + 1] : 0, 1, k < maxit ? 1 : 0, maxit, cap};
+        const LoopCtl lc{k < maxit ? hc[k] : 0, k < maxit ? hm[k + 1] : 0, 1, k < maxit ? 1 : 0, maxit, cap,
+                         I.chain_nc, ctx->order == AMCFD_ORDER_EXACT};
         if (q) swap_props<T>(I);
         cudaGraph_t tail = capture([&] {
             run_phase_impl<T>(ctx, I, AMCFD_PHASE_SPECIES);

@@ -55,8 +55,8 @@ struct Status {
     // per step
     double timet, delt, beamposx, beamposy, scanvel;
     // device-driven outer loop: iterations run in this step, momentum-box cells of
-    // the last one (-1: none yet), momentum path of the current one (1: small box)
-    // and iterations that took the small-box path
+    // the last one (-1: none yet), momentum path of the current one (1: small box;
+    // the host sets the first iteration's) and iterations that took the small-box path
     int lp_niter, lp_box, lp_mode, lp_small;
     int powerindicator, istart, jstart, heat_iter;
     double heatinlaser;
@@ -92,6 +92,7 @@ struct Status {
 struct LoopCtl {
     cudaGraphConditionalHandle cont, mode_next;
     int active, has_next, maxit, cap;  // cap: small-box capacity in cells, -1 when disabled
+    int chain_nc, exact;               // one-launch chain: its cluster size (0: not used), the exact order
 };
 
 // Fixed-size reduction slots written per CTA and reduced in a fixed order.

@@ -692,7 +692,10 @@ __global__ void converge_kernel(Params p, Fields<T> gd, const double *red_h2t, i
             st->lp_small += st->lp_mode;
             const int box = st->momentum_active ? st->box_cells : 0;
             st->lp_box = box;
-            const int mode = lc.cap >= 0 && box <= lc.cap;
+            const int mode = lc.chain_nc > 0
+                ? (!st->momentum_active || chain_box_fits(st->iendm1 - st->istatp1 + 1, st->jend - st->jstat + 1,
+                                                          p.nkm2 - st->kstat + 1, lc.exact, lc.chain_nc))
+                : lc.cap >= 0 && box <= lc.cap;
             st->lp_mode = mode;
             const int cont = !conv && !st->nonfinite && !*(volatile int *)&st->error && it < lc.maxit;
             if (lc.has_next) {
@@ -705,12 +708,10 @@ __global__ void converge_kernel(Params p, Fields<T> gd, const double *red_h2t, i
 }
 
 // Head of a step captured as one graph: the momentum path of its first outer
-// iteration, from the box of the last iteration before it.
+// iteration, which the host has chosen from the box of the last iteration before it.
 __global__ void loop_init_kernel(Status *st, LoopCtl lc)
 {
-    const int mode = lc.cap >= 0 && st->lp_box >= 0 && st->lp_box <= lc.cap;
-    st->lp_mode = mode;
-    cudaGraphSetConditional(lc.mode_next, (unsigned)mode);
+    cudaGraphSetConditional(lc.mode_next, (unsigned)st->lp_mode);
 }
 void launch_loop_init(Status *st, const LoopCtl &lc, cudaStream_t s)
 {

@@ -38,6 +38,17 @@ __device__ __forceinline__ void box_cell(const Box &b, int q, int &i, int &j, in
     k = b.k0 + r / b.nj_;
 }
 
+// Reads of a field that other CTAs may have written: through L2 only inside a
+// launch that also writes the field (LdL2), plain loads otherwise (LdPlain).
+template <typename T> struct LdPlain {
+    const T *p;
+    __device__ __forceinline__ T operator[](size_t c) const { return p[c]; }
+};
+template <typename T> struct LdL2 {
+    const T *p;
+    __device__ __forceinline__ T operator[](size_t c) const { return __ldcg(p + c); }
+};
+
 // cleanVelocities (CFDSolverManager.cpp:2577-2620), one box cell.
 template <typename T>
 __device__ __forceinline__ void clean_cell(const Params &p, const Fields<T> &g, int i, int j, int k)
@@ -86,7 +97,7 @@ __device__ __forceinline__ int mom_bc_items(const Params &p, const Status *st, c
     ntop = (ivar <= 2) ? b.ni_ * b.nj_ : 0;
     return ntop + b.nj_ * (p.nkm1 - b.k0);
 }
-template <typename T>
+template <typename T, class LD = LdPlain<T>>
 __device__ __forceinline__ double mom_bc_item(const Params &p, const Fields<T> &g, const Status *st,
                                               const Box &b, int ivar, int q, int ntop)
 {
@@ -112,7 +123,7 @@ __device__ __forceinline__ double mom_bc_item(const Params &p, const Fields<T> &
         }
         double term1 = fl * surface_tension_gradient(tt, p.a_oxygen, p.dgdtp) * grad /
                        (vis1 * g.dzpbinv[nkm1]);
-        T val = (T)((double)phi[cb] + term1);
+        T val = (T)((double)LD{phi}[cb] + term1);
         phi[ct] = val;
         return ivar == 1 ? fabs((double)val) : 0.0;
     }
@@ -143,25 +154,31 @@ __global__ void mom_bc_kernel(Params p, Fields<T> g, int ivar, double *red_umax)
     }
 }
 
+// The equation of one box cell: its coefficients, the unknown on the four
+// neighbouring lines (top, bottom, north, south) and d = A/ap.
+template <typename T> struct CellEq {
+    T an, as, ae, aw, at, ab, ap, su, d, pt, pb, pn, ps;
+};
+
 // One cell of the u/v/w equation (ivar 1..3) of the momentum box: coefficients,
-// source, under-relaxation, the solid freeze and d = A/ap, written to the shared
-// coefficient arrays; returns |residual| of the cell (calculateResiduals(1..3)).
-template <typename T>
-__device__ __forceinline__ double mom_assemble_cell(const Params &p, const Fields<T> &g, const Status *st,
-                                                    int ivar, int i, int j, int k)
+// source, under-relaxation, the solid freeze and d = A/ap; returns |residual| of
+// the cell (calculateResiduals(1..3)).
+template <typename T, class LD>
+__device__ __forceinline__ double mom_cell_eq(const Params &p, const Fields<T> &g, const Status *st, int ivar, int i,
+                                              int j, int k, CellEq<T> &q)
 {
     using R = T;
     const int nj = p.nj, nip = p.nip, nkm2 = p.nkm2, njm2 = p.njm2, nim2 = p.nim2;
     const size_t sj = nip, sk = (size_t)nj * nip;
     const int sch = p.scheme;
     const R delt = (R)st->delt;
-    const R *u = g.uvel, *v = g.vvel, *w = g.wvel, *rho = g.rho_nxt, *vis = g.vis_nxt;
+    const LD u{g.uvel}, v{g.vvel}, w{g.wvel};
+    const R *rho = g.rho_nxt, *vis = g.vis_nxt;
     const double *fx = g.fracx, *fy = g.fracy, *fz = g.fracz, *xu = g.xu, *yv = g.yv, *zw = g.zw;
     const size_t c = cidx(i, j, k, nj, nip);
     R an, as_, ae, aw, at, ab, apnot, su, sp, tmp, areaD, vol;
     const R rc = rho[c];
-    R *phi;
-    const R *phinot;
+    LD phi;
     size_t cn;  // upstream scalar node of the staggered cell
     R urf, flv;
     if (ivar == 1) {
@@ -211,7 +228,7 @@ __device__ __forceinline__ double mom_assemble_cell(const Params &p, const Field
         R dwdxp = (w[c + sk] - w[c + sk - 1]) * (R)g.dxpwinv[i];
         R dwdxm = (w[c] - w[c - 1]) * (R)g.dxpwinv[i];
         su += (vist * dwdxp - visb * dwdxm) * auij;
-        phi = g.uvel; phinot = g.unot; cn = c - 1; urf = (R)p.urfu; areaD = ajk;
+        phi = u; cn = c - 1; urf = (R)p.urfu; areaD = ajk;
         flv = g.fracl[c] * (R(1) - fxm) + g.fracl[c - 1] * fxm;
     } else if (ivar == 2) {
         const R fym = (R)fy[j - 1];
@@ -260,7 +277,7 @@ __device__ __forceinline__ double mom_assemble_cell(const Params &p, const Field
         R dwdyp = (w[c + sk] - w[c + sk - sj]) * (R)g.dypsinv[j];
         R dwdym = (w[c] - w[c - sj]) * (R)g.dypsinv[j];
         su += (vist * dwdyp - visb * dwdym) * avij;
-        phi = g.vvel; phinot = g.vnot; cn = c - sj; urf = (R)p.urfv; areaD = aik;
+        phi = v; cn = c - sj; urf = (R)p.urfv; areaD = aik;
         flv = g.fracl[c] * (R(1) - fym) + g.fracl[c - sj] * fym;
     } else {
         const R fzm = (R)fz[k - 1];
@@ -309,10 +326,9 @@ __device__ __forceinline__ double mom_assemble_cell(const Params &p, const Field
         R dwdzp = (w[c + sk] - w[c]) / (R)(zw[k + 1] - zw[k]);
         R dwdzm = (w[c] - w[c - sk]) / (R)(zw[k] - zw[k - 1]);
         su += (vist * dwdzp - visb * dwdzm) * aij;
-        phi = g.wvel; phinot = g.wnot; cn = c - sk; urf = (R)p.urfw; areaD = aij;
+        phi = w; cn = c - sk; urf = (R)p.urfw; areaD = aij;
         flv = g.fracl[c] * (R(1) - fzm) + g.fracl[c - sk] * fzm;
     }
-    (void)phinot;
     // ---- calculateSource ----
     if (flv > R(0)) {
         R term = (R)p.darcyKo * ((R(1) - flv) * (R(1) - flv)) / ((flv * flv * flv) + (R)kSmall);
@@ -344,12 +360,29 @@ __device__ __forceinline__ double mom_assemble_cell(const Params &p, const Field
         an = as_ = ae = aw = at = ab = R(0);
         ap = (R)kLarge;
     }
-    g.an[c] = an; g.as[c] = as_; g.ae[c] = ae; g.aw[c] = aw; g.at[c] = at; g.ab[c] = ab;
-    g.ap[c] = ap; g.su[c] = su;
-    (ivar == 1 ? g.dux : ivar == 2 ? g.dvy : g.dwz)[c] = dcoef;
-    R r = an * phi[c + sj] + as_ * phi[c - sj] + ae * phi[c + 1] + aw * phi[c - 1] +
-          at * phi[c + sk] + ab * phi[c - sk] + su - ap * phi[c];
+    q.an = an; q.as = as_; q.ae = ae; q.aw = aw; q.at = at; q.ab = ab; q.ap = ap; q.su = su; q.d = dcoef;
+    q.pt = phi[c + sk]; q.pb = phi[c - sk]; q.pn = phi[c + sj]; q.ps = phi[c - sj];
+    R r = an * q.pn + as_ * q.ps + ae * phi[c + 1] + aw * phi[c - 1] + at * q.pt + ab * q.pb + su - ap * phi[c];
     return fabs((double)r);
+}
+
+// The coefficients of cell c into the shared coefficient arrays.
+template <typename T>
+__device__ __forceinline__ void store_cell_eq(const Fields<T> &g, size_t c, const CellEq<T> &q)
+{
+    g.an[c] = q.an; g.as[c] = q.as; g.ae[c] = q.ae; g.aw[c] = q.aw; g.at[c] = q.at; g.ab[c] = q.ab;
+    g.ap[c] = q.ap; g.su[c] = q.su;
+}
+template <typename T>
+__device__ __forceinline__ double mom_assemble_cell(const Params &p, const Fields<T> &g, const Status *st,
+                                                    int ivar, int i, int j, int k)
+{
+    CellEq<T> q;
+    const double r = mom_cell_eq<T, LdPlain<T>>(p, g, st, ivar, i, j, k, q);
+    const size_t c = cidx(i, j, k, p.nj, p.nip);
+    store_cell_eq<T>(g, c, q);
+    (ivar == 1 ? g.dux : ivar == 2 ? g.dvy : g.dwz)[c] = q.d;
+    return r;
 }
 
 // discretizeEquations(1..3) + calculateSource(1..3) + calculateResiduals(1..3)
@@ -376,23 +409,23 @@ __global__ void __launch_bounds__(256) mom_assemble_kernel(Params p, Fields<T> g
 // discretizeEquations(4) + calculateSource(4) + calculateResiduals(4)
 // (CFDSolverManager.cpp:1112-1156, 1645-1676, 2047-2071), one box cell: p'
 // coefficients, |mass imbalance| and the mass-flux denominator added to the sums.
-template <typename T>
-__device__ __forceinline__ void pp_assemble_cell(const Params &p, const Fields<T> &g, int i, int j, int k,
-                                                 double &resorm, double &denom)
+template <typename T, class LD>
+__device__ __forceinline__ void pp_cell_eq(const Params &p, const Fields<T> &g, int i, int j, int k, CellEq<T> &q,
+                                           double &resorm, double &denom)
 {
     using R = T;
     const int nj = p.nj, nip = p.nip;
     const size_t sj = nip, sk = (size_t)nj * nip;
-    const R *u = g.uvel, *v = g.vvel, *w = g.wvel, *rho = g.rho_nxt;
+    const LD u{g.uvel}, v{g.vvel}, w{g.wvel}, dux{g.dux}, dvy{g.dvy}, dwz{g.dwz};
     const size_t c = cidx(i, j, k, nj, nip);
-    const R rc = rho[c];
+    const R rc = g.rho_nxt[c];
     const R aik = (R)area_ik(p, g, i, k), ajk = (R)area_jk(p, g, j, k), aij = (R)area_ij(p, g, i, j);
-    R an = aik * g.dvy[c + sj] * rc;
-    R as_ = aik * g.dvy[c] * rc;
-    R ae = ajk * g.dux[c + 1] * rc;
-    R aw = ajk * g.dux[c] * rc;
-    R at = aij * g.dwz[c + sk] * rc;
-    R ab = aij * g.dwz[c] * rc;
+    R an = aik * dvy[c + sj] * rc;
+    R as_ = aik * dvy[c] * rc;
+    R ae = ajk * dux[c + 1] * rc;
+    R aw = ajk * dux[c] * rc;
+    R at = aij * dwz[c + sk] * rc;
+    R ab = aij * dwz[c] * rc;
     R fn = v[c + sj] * aik * rc, fs = v[c] * aik * rc;
     R fe = u[c + 1] * ajk * rc, fw = u[c] * ajk * rc;
     R ft = w[c + sk] * aij * rc, fb = w[c] * aij * rc;
@@ -405,12 +438,19 @@ __device__ __forceinline__ void pp_assemble_cell(const Params &p, const Fields<T
         an = as_ = ae = aw = at = ab = R(0);
         ap = (R)kLarge;
     }
-    g.an[c] = an; g.as[c] = as_; g.ae[c] = ae; g.aw[c] = aw; g.at[c] = at; g.ab[c] = ab;
-    g.ap[c] = ap; g.su[c] = su;
+    q.an = an; q.as = as_; q.ae = ae; q.aw = aw; q.at = at; q.ab = ab; q.ap = ap; q.su = su;
     double dtp = (fabs((double)u[c]) + fabs((double)u[c + 1])) * (double)ajk +
                  (fabs((double)v[c]) + fabs((double)v[c + sj])) * (double)aik +
                  (fabs((double)w[c]) + fabs((double)w[c + sk])) * (double)aij;
     denom += 0.5 * fabs(dtp);
+}
+template <typename T>
+__device__ __forceinline__ void pp_assemble_cell(const Params &p, const Fields<T> &g, int i, int j, int k,
+                                                 double &resorm, double &denom)
+{
+    CellEq<T> q;
+    pp_cell_eq<T, LdPlain<T>>(p, g, i, j, k, q, resorm, denom);
+    store_cell_eq<T>(g, cidx(i, j, k, p.nj, p.nip), q);
 }
 template <typename T>
 __global__ void __launch_bounds__(256) pp_assemble_kernel(Params p, Fields<T> g, double *red)
@@ -433,24 +473,25 @@ __global__ void __launch_bounds__(256) pp_assemble_kernel(Params p, Fields<T> g,
 
 // correctPressure (CFDSolverManager.cpp:2692-2758): velocity correction, then
 // pressure update (two passes: the second zeroes p' that the first reads).
-template <typename T>
+template <typename T, class LD = LdPlain<T>>
 __device__ __forceinline__ void correct_velocity_cell(const Params &p, const Fields<T> &g, int i, int j, int k)
 {
     const int nj = p.nj, nip = p.nip;
     const size_t sj = nip, sk = (size_t)nj * nip;
     const T ts = (T)p.tsolid;
     size_t c = cidx(i, j, k, nj, nip);
-    T tc = g.temp[c], ppc = g.pp[c];
-    if (mind(tc, g.temp[c - 1]) > ts) g.uvel[c] += g.dux[c] * (g.pp[c - 1] - ppc);
-    if (mind(tc, g.temp[c - sj]) > ts) g.vvel[c] += g.dvy[c] * (g.pp[c - sj] - ppc);
-    if (mind(tc, g.temp[c - sk]) > ts) g.wvel[c] += g.dwz[c] * (g.pp[c - sk] - ppc);
+    const LD pp{g.pp}, u{g.uvel}, v{g.vvel}, w{g.wvel}, dux{g.dux}, dvy{g.dvy}, dwz{g.dwz};
+    T tc = g.temp[c], ppc = pp[c];
+    if (mind(tc, g.temp[c - 1]) > ts) g.uvel[c] = u[c] + dux[c] * (pp[c - 1] - ppc);
+    if (mind(tc, g.temp[c - sj]) > ts) g.vvel[c] = v[c] + dvy[c] * (pp[c - sj] - ppc);
+    if (mind(tc, g.temp[c - sk]) > ts) g.wvel[c] = w[c] + dwz[c] * (pp[c - sk] - ppc);
 }
-template <typename T>
+template <typename T, class LD = LdPlain<T>>
 __device__ __forceinline__ void correct_pressure_cell(const Params &p, const Fields<T> &g, int i, int j, int k)
 {
     size_t c = cidx(i, j, k, p.nj, p.nip);
     if (g.temp[c] > (T)p.tsolid) {
-        g.pressure[c] += (T)p.urfp * g.pp[c];
+        g.pressure[c] += (T)p.urfp * LD{g.pp}[c];
         g.pp[c] = T(0);
     }
 }
@@ -1627,6 +1668,561 @@ mom_cluster_post_kernel(Params p, Fields<T> g, T *scratch, int smem_elems, const
     }
 }
 
+// ---------------------------------------------------------------------------
+// The whole momentum chain of an outer iteration (iterativeLoopSolve,
+// CFDSolverManager.cpp:660-675) in one launch: one cluster of CTAs takes the box
+// through cleanVelocities, then per equation applyBCs, the coefficient assembly,
+// the line factorisation and the four visits of every line, and for p'
+// correctPressure and the residual normalisation.
+//
+// What bounds it: latency.  The box holds 1000-6000 cells in lines of 10-40; as
+// ten launches (two per equation and two before them, lines exchanging values
+// through L2) the chain took 94 us an outer iteration in FP32 and 150 in FP64,
+// of which the arithmetic is a few us: launch and drain gaps, the coefficients'
+// round trip through global memory, and an L2 round trip of about 1.2 us for
+// each of the 8 x 4 dependent colour passes.  Here
+//   * a warp owns one line (two where the box has more lines than the cluster
+//     warps) and assembles that line's cells itself, so coefficients and
+//     factorisation never leave its shared memory;
+//   * a line's new values are pushed straight into the shared memory of the
+//     (up to four) lines that read them, on whichever CTA of the cluster they
+//     live, by st.async: the stores complete on the receiving line's mbarrier, so
+//     a value and the news of it travel together in one hop;
+//   * launches become cluster barriers (0.2 us measured).
+// The arithmetic is that of the multi-launch chain operation for operation
+// (line_rhs, the scans of solve_line_regs, factor_cell; the residual sums are
+// formed from per-cell values in the order of its per-CTA partials), so both give
+// the same bits, in red-black and in the reference's order.
+//
+// Visits.  A line is solved four times (2 k-sweeps x 2 j-sweeps).  Visit v of a
+// line may run once the lines it reads have reached the values it is to read:
+//   red-black, colour c (visit v is pass 2v + c): the four neighbours' previous
+//     pass, none for the very first pass;
+//   exact order, v = 2 ks + s: (j-1) visit v; (j+1) visit v-1; for s = 0 (k+1)
+//     visit v+1 and, for v = 2, (k-1) visit 1.
+// A neighbour pushes exactly those values.  Every push for visit v depends on this
+// line's visit v-1, so one mailbox per direction is enough and the transactions
+// of two visits never share an mbarrier phase.  A warp with two lines runs
+// their visits in the order of the pass (exact order: of the wave
+// t = 3m + (j-j0) + 2s of k_linesolve.cu), which every dependency precedes.
+// A wait that runs out (wait_polls) records AMCFD_E_TIMEOUT and the launch goes on
+// without waiting: no CTA leaves while another may still push to it.
+//
+// A box that has outgrown the lines' shared memory since the launch was chosen
+// (kChainLines lines a CTA, kChainCells cells a line) is solved in place in
+// global memory by the same warps, cluster barriers between the passes.
+// ---------------------------------------------------------------------------
+constexpr int kChainThreads = 512;
+enum { C_AT = 0, C_AB, C_AN, C_AS, C_SU, C_CF, C_PR, C_ID, C_N };  // coefficient rows of a line
+enum { D_T = 0, D_B, D_N, D_S };                                   // mailbox directions: k+1, k-1, j+1, j-1
+
+template <typename T> struct ChainLine {
+    T coef[C_N][kChainCells];
+    T mail[4][kChainCells];
+    T lo, hi;
+};
+struct ChainInfo {
+    unsigned long long bar;
+    unsigned nmail[4], nbar[4];  // shared::cluster addresses in the four neighbours (their mailbox, their mbarrier)
+    int j, k, in;                // in: bit d set when the neighbour in direction d lies in the box; j < 0: no line
+};
+
+__device__ __forceinline__ void cluster_barrier()
+{
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ unsigned map_rank(unsigned addr, unsigned rank)
+{
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_async(unsigned addr, unsigned bar, float v)
+{
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr),
+                 "r"(__float_as_uint(v)), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void st_async(unsigned addr, unsigned bar, double v)
+{
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr),
+                 "l"(__double_as_longlong(v)), "r"(bar) : "memory");
+}
+// Bounded wait of the whole warp on phase `parity`, with cluster-scope acquire.
+__device__ __forceinline__ bool chain_wait(unsigned bar, unsigned parity, Status *st, long long polls)
+{
+    for (long long it = 0;; ++it) {
+        unsigned done;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+            " selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+        if (__all_sync(0xffffffffu, done)) return true;
+        if ((it & 63) == 63 && __any_sync(0xffffffffu, *(volatile int *)&st->error != 0)) return false;
+        if (it > polls) {
+            if ((threadIdx.x & 31) == 0 && atomicCAS(&st->error, 0, AMCFD_E_TIMEOUT) == 0) st->error_where = -6;
+            return false;
+        }
+    }
+}
+
+// Directions whose values visit v of a line waits for, among its in-box neighbours,
+// and those it pushes to after the visit.
+template <bool EXACT>
+__device__ __forceinline__ int chain_waits(int v, int c, int in)
+{
+    if (EXACT) return in & ((1 << D_S) | (v >= 1 ? 1 << D_N : 0) | ((v & 1) == 0 ? 1 << D_T : 0) | (v == 2 ? 1 << D_B : 0));
+    return (c == 0 && v == 0) ? 0 : in;
+}
+template <bool EXACT>
+__device__ __forceinline__ int chain_pushes(int v, int c, int in)
+{
+    if (EXACT) return in & ((1 << D_N) | (v < 3 ? 1 << D_S : 0) | ((v & 1) ? 1 << D_B : 0) | (v == 1 ? 1 << D_T : 0));
+    return (c == 1 && v == 3) ? 0 : in;
+}
+// In-box directions whose first value is pushed by the neighbour (the others
+// start from the unknown's value before the solve).
+template <bool EXACT>
+__device__ __forceinline__ int chain_first_pushed(int c, int in)
+{
+    if (EXACT) return in & ((1 << D_S) | (1 << D_T));
+    return c == 1 ? in : 0;
+}
+
+// One visit of a line of n <= 32 L cells from its shared memory: solve_line_regs
+// with the neighbours' values from the mailboxes; `to` the directions to push to.
+template <typename T, int L>
+__device__ __forceinline__ void chain_visit(ChainLine<T> &ln, const ChainInfo &inf, int n, int to, T *out)
+{
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int a = lane * L;
+    T e[L], cf[L], pr[L];
+#pragma unroll
+    for (int v = 0; v < L; ++v) {
+        const int q = a + v < n ? a + v : 0;
+        e[v] = line_rhs(ln.coef[C_AT][q], ln.mail[D_T][q], ln.coef[C_AB][q], ln.mail[D_B][q], ln.coef[C_AN][q],
+                        ln.mail[D_N][q], ln.coef[C_AS][q], ln.mail[D_S][q], ln.coef[C_SU][q], ln.coef[C_ID][q]);
+        cf[v] = ln.coef[C_CF][q];
+        pr[v] = ln.coef[C_PR][q];
+    }
+    T A = T(1), B = T(0);
+#pragma unroll
+    for (int v = 0; v < L; ++v)
+        if (a + v < n) {
+            B = fma_rn(cf[v], B, e[v]);
+            A = mul_rn(cf[v], A);
+        }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const T A2 = __shfl_up_sync(full, A, o), B2 = __shfl_up_sync(full, B, o);
+        if (lane >= o) {
+            B = fma_rn(A, B2, B);
+            A = mul_rn(A, A2);
+        }
+    }
+    T Ae = __shfl_up_sync(full, A, 1), Be = __shfl_up_sync(full, B, 1);
+    if (lane == 0) { Ae = T(1); Be = T(0); }
+    T x = fma_rn(Ae, ln.lo, Be);
+#pragma unroll
+    for (int v = 0; v < L; ++v)
+        if (a + v < n) {
+            x = fma_rn(cf[v], x, e[v]);
+            e[v] = x;
+        }
+    A = T(1);
+    B = T(0);
+#pragma unroll
+    for (int v = L - 1; v >= 0; --v)
+        if (a + v < n) {
+            B = fma_rn(pr[v], B, e[v]);
+            A = mul_rn(pr[v], A);
+        }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const T A2 = __shfl_down_sync(full, A, o), B2 = __shfl_down_sync(full, B, o);
+        if (lane + o < 32) {
+            B = fma_rn(A, B2, B);
+            A = mul_rn(A, A2);
+        }
+    }
+    Ae = __shfl_down_sync(full, A, 1);
+    Be = __shfl_down_sync(full, B, 1);
+    if (lane == 31) { Ae = T(1); Be = T(0); }
+    x = fma_rn(Ae, ln.hi, Be);
+#pragma unroll
+    for (int v = L - 1; v >= 0; --v)
+        if (a + v < n) {
+            x = fma_rn(pr[v], x, e[v]);
+#pragma unroll
+            for (int d = 0; d < 4; ++d)
+                if (to >> d & 1) st_async(inf.nmail[d] + (unsigned)((a + v) * sizeof(T)), inf.nbar[d], x);
+            if (out) out[a + v] = x;
+        }
+}
+
+// The serial factorisation of the reference's order (factor_kernel<T, true>), one
+// lane, through accessors as factor_line_mem's.
+template <typename T, class Get, class Put>
+__device__ __forceinline__ void factor_line_serial(int n, Get get, Put put)
+{
+    T x = T(0);
+    for (int i = 0; i < n; ++i) {
+        T w, e, p, pr, cf, id;
+        get(i, w, e, p);
+        factor_cell(w, e, p, x, pr, cf, id);
+        put(i, pr, cf, id);
+    }
+}
+
+// One visit of a line in place in global memory (solve_staged's operations; the
+// right-hand side and the recurrences in `scratch`).
+template <typename T>
+__device__ void chain_visit_mem(const Fields<T> &g, T *phi, T *scratch, size_t row, int i0, int i1, size_t sj,
+                                size_t sk)
+{
+    const int lane = threadIdx.x & 31;
+    const T lo = __ldcg(phi + row + i0 - 1), hi = __ldcg(phi + row + i1 + 1);
+    for (int i = i0 + lane; i <= i1; i += 32) {
+        const size_t c = row + i;
+        scratch[c] = line_rhs(g.at[c], __ldcg(phi + c + sk), g.ab[c], __ldcg(phi + c - sk), g.an[c],
+                              __ldcg(phi + c + sj), g.as[c], __ldcg(phi + c - sj), g.su[c], g.iden[c]);
+    }
+    __syncwarp();
+    scan_line<T>(phi, row, i0, i1, scratch + row + i0, g.cf + row + i0, g.pr + row + i0, lo, hi);
+    __syncwarp();
+}
+
+// mom_finalize_body of the chain's last CTA, a warp per sum (nb <= 128 partials: the
+// sums of the 32-entry groups by warp trees and a tree over them, the order of
+// reduce_sums); scr holds 8 doubles.
+__device__ __forceinline__ void chain_finalize(const Params &p, Status *st, const double *red, int nb, int nb_umax,
+                                               int nb_region, double *scr)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp < 6) {
+        const int region = warp < 3 ? warp : warp == 5 ? 4 : 3;
+        const int slot = warp < 3 ? R_MSUMD : warp == 3 ? R_MRESORM : warp == 4 ? R_MDENOM : R_UMAX;
+        const int m = warp == 5 ? nb_umax : nb;
+        double x[4], y = warp == 5 ? -INFINITY : 0.0;
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            const int q = v * 32 + lane;
+            x[v] = q < m ? __ldcg(red + ((size_t)region * nb_region + q) * R_NSLOTS + slot) : y;
+        }
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            const double z = warp == 5 ? warp_max(x[v]) : warp_sum(x[v]);
+            if (lane == v) y = z;
+        }
+        y = warp == 5 ? warp_max(y) : warp_sum(y);
+        if (lane == 0) scr[warp] = y;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) mom_finalize_status(p, st, scr[0], scr[1], scr[2], scr[3], scr[4], scr[5]);
+}
+
+template <typename T> size_t chain_smem() { return kChainLines * (sizeof(ChainLine<T>) + sizeof(ChainInfo)); }
+
+template <typename T, bool EXACT>
+__global__ void __launch_bounds__(kChainThreads, 1)
+mom_chain_kernel(Params p, Fields<T> g, double *red, int nb_region, double *rcell, int rcap, T *scratch)
+{
+    pdl_enter();
+    extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ double sh[40];
+    ChainLine<T> *lines = reinterpret_cast<ChainLine<T> *>(smraw);
+    ChainInfo *info = reinterpret_cast<ChainInfo *>(smraw + kChainLines * sizeof(ChainLine<T>));
+    Status *st = g.st;
+    Box b;
+    // the same decision in every thread: nothing sets the error before the first barrier
+    if (!get_box(st, p, b) || *(volatile int *)&st->error) return;
+    unsigned rank, nc;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(nc));
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = kChainThreads / 32;
+    const int t = (int)rank * kChainThreads + threadIdx.x, nt = (int)nc * kChainThreads;
+    const int i0 = b.i0, i1 = b.i1, j0 = b.j0, j1 = b.j1, k0 = b.k0, k1 = b.k1;
+    const int n = b.ni_, J = b.nj_, K = k1 - k0 + 1, nj = p.nj, nip = p.nip;
+    const size_t sj = nip, sk = (size_t)nj * nip;
+    // line slots: exact order, every (k, j); red-black, pairs of one line of each colour
+    const int half = (J + 1) / 2, nl = EXACT ? J * K : 2 * half * K;
+    const int lpc = (nl + (int)nc - 1) / (int)nc;  // a CTA's share
+    using LD = LdL2<T>;
+    const bool fits = n <= kChainCells && lpc <= kChainLines && b.n <= rcap;
+    // slot -> line; false where the slot holds none
+    auto slot_line = [&](int l, int &j, int &k) {
+        if (EXACT) {
+            k = k0 + l / J;
+            j = j0 + l % J;
+            return l < nl;
+        }
+        const int q = l >> 1, kk = q / half;
+        k = k0 + kk;
+        j = j0 + (((l & 1) - k - j0) % 2 + 2) % 2 + 2 * (q - kk * half);
+        return l < nl && j <= j1;
+    };
+    auto line_slot = [&](int j, int k) {
+        if (EXACT) return (k - k0) * J + j - j0;
+        const int c = (j + k) & 1;
+        return 2 * ((k - k0) * half + (j - j0) / 2) + c;
+    };
+    const int first = (int)rank * lpc, nloc = max(0, min(lpc, nl - first));
+    if (fits && (int)threadIdx.x < nloc) {
+        ChainInfo &f = info[threadIdx.x];
+        int j, k;
+        if (slot_line(first + threadIdx.x, j, k)) {
+            f.in = (k < k1 ? 1 << D_T : 0) | (k > k0 ? 1 << D_B : 0) | (j < j1 ? 1 << D_N : 0) | (j > j0 ? 1 << D_S : 0);
+            const int dj[4] = {0, 0, 1, -1}, dk[4] = {1, -1, 0, 0}, back[4] = {D_B, D_T, D_S, D_N};
+            for (int d = 0; d < 4; ++d) {
+                if (!(f.in >> d & 1)) continue;
+                const int l = line_slot(j + dj[d], k + dk[d]), r = l / lpc;
+                f.nmail[d] = map_rank(smem_u32(&lines[l - r * lpc].mail[back[d]][0]), (unsigned)r);
+                f.nbar[d] = map_rank(smem_u32(&info[l - r * lpc].bar), (unsigned)r);
+            }
+            f.j = j;
+        } else {
+            f.j = -1;
+        }
+        f.k = k;
+        mbar_init(reinterpret_cast<uint64_t *>(&f.bar));
+    }
+    // the rows the first assembly reads start towards L2 (a deck past the L2's
+    // capacity has evicted them since the iteration before), a field a lane
+    {
+        const T *src[16] = {g.uvel, g.vvel, g.wvel, g.pressure, g.vis_nxt, g.rho_nxt, g.unot, g.vnot,
+                            g.wnot, g.fracl, g.pp,  g.dux,      g.dvy,     g.dwz,     g.temp, g.temp};
+        for (int l = warp; l < nloc; l += nw) {
+            int j, k;
+            if (!slot_line(first + l, j, k)) continue;
+            const T *row = src[0];
+#pragma unroll
+            for (int a = 1; a < 16; ++a)
+                if ((lane & 15) == a) row = src[a];
+            row += cidx(lane < 16 ? i0 - 1 : i0 + n, j, k, nj, nip);
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(row));
+        }
+    }
+    for (int q = t; q < b.n; q += nt) {
+        int i, j, k;
+        box_cell(b, q, i, j, k);
+        clean_cell<T>(p, g, i, j, k);
+    }
+    __syncthreads();
+    cluster_barrier();
+    {
+        int ntop;
+        const int nbc = mom_bc_items(p, st, b, 1, ntop);
+        double um = 0.0;
+        for (int q = t; q < nbc; q += nt) um = maxd(um, mom_bc_item<T, LD>(p, g, st, b, 1, q, ntop));
+        um = cta_max(um, sh);
+        if (threadIdx.x == 0) red[((size_t)4 * nb_region + rank) * R_NSLOTS + R_UMAX] = um;
+    }
+    __syncwarp();
+    cluster_barrier();
+    unsigned par = 0;  // phase parities of the warp's two lines
+    bool ok = true;
+    const bool cells = b.n <= rcap;  // per-cell residuals kept (else per-CTA sums, in another order)
+    const int nblk = cells ? (b.n + 255) / 256 : 0;
+    // Work of equation `iv` beside its visits, spread over `nh` threads from `h`: the
+    // boundary values of the next equation, and the residual sums in the order of
+    // the multi-launch assemblies (blocks of 256 box cells: eight warp trees and a
+    // tree over them).  It needs every line's assembly of the equation done.
+    auto beside = [&](int iv, int h, int nh) {
+        if (iv <= 3) {
+            int ntop;
+            const int nbc = mom_bc_items(p, st, b, iv + 1, ntop);
+            for (int q = h; q < nbc; q += nh) mom_bc_item<T, LD>(p, g, st, b, iv + 1, q, ntop);
+        }
+        __syncwarp();
+        for (int q = h >> 5; q < (iv == 4 ? 2 : 1) * nblk; q += nh >> 5) {
+            const int blk = q % nblk, e = iv - 1 + q / nblk;
+            double x[8], y = 0.0;
+#pragma unroll
+            for (int v = 0; v < 8; ++v) {
+                const int c = blk * 256 + v * 32 + lane;
+                x[v] = c < b.n ? __ldcg(rcell + (size_t)e * rcap + c) : 0.0;
+            }
+#pragma unroll
+            for (int v = 0; v < 8; ++v) x[v] = warp_sum(x[v]);
+#pragma unroll
+            for (int v = 0; v < 8; ++v)
+                if (lane == v) y = x[v];
+            y = warp_sum(y);
+            if (lane == 0)
+                red[((size_t)(iv - 1) * nb_region + blk) * R_NSLOTS +
+                    (iv <= 3 ? R_MSUMD : e == 3 ? R_MRESORM : R_MDENOM)] = y;
+        }
+        __syncwarp();
+    };
+    // the warps without a line do that while the others visit theirs (the first CTAs
+    // of a box with fewer lines than warps have some); otherwise every warp does it
+    // after its visits
+    const int idle = fits && lpc < nw ? nw - lpc : 0;
+#pragma unroll 1
+    for (int ivar = 1; ivar <= 4; ++ivar) {
+        T *phi = ivar == 1 ? g.uvel : ivar == 2 ? g.vvel : ivar == 3 ? g.wvel : g.pp;
+        // ---- assembly and factorisation of this warp's lines ----
+        double sum = 0.0, sumd = 0.0;
+#pragma unroll 1
+        for (int l = warp; l < nloc; l += nw) {
+            int j, k;
+            if (!slot_line(first + l, j, k)) continue;
+            const size_t row = cidx(i0, j, k, nj, nip);
+            ChainLine<T> &ln = lines[fits ? l : 0];
+            int fill = 0;
+            if (fits) {
+                const int in = info[l].in;
+                fill = 0xf & ~chain_first_pushed<EXACT>((j + k) & 1, in);
+                if (lane == 0) {
+                    ln.lo = __ldcg(phi + row - 1);
+                    ln.hi = __ldcg(phi + row + n);
+                }
+            }
+#pragma unroll 1
+            for (int i = lane; i < n; i += 32) {
+                CellEq<T> q;
+                const size_t c = row + i;
+                const size_t qc = (size_t)((k - k0) * J + j - j0) * n + i;  // box-cell order
+                double r, rd = 0.0;
+                if (ivar <= 3) {
+                    r = mom_cell_eq<T, LD>(p, g, st, ivar, i0 + i, j, k, q);
+                    (ivar == 1 ? g.dux : ivar == 2 ? g.dvy : g.dwz)[c] = q.d;
+                } else {
+                    r = 0.0;
+                    pp_cell_eq<T, LD>(p, g, i0 + i, j, k, q, r, rd);
+                    q.pt = __ldcg(phi + c + sk); q.pb = __ldcg(phi + c - sk);
+                    q.pn = __ldcg(phi + c + sj); q.ps = __ldcg(phi + c - sj);
+                }
+                if (cells) {
+                    rcell[(size_t)(ivar - 1) * rcap + qc] = r;
+                    if (ivar == 4) rcell[(size_t)4 * rcap + qc] = rd;
+                } else {
+                    sum += r;
+                    sumd += rd;
+                }
+                // the coefficient arrays end as the chain's last equation leaves them
+                if (ivar == 4 || !fits) store_cell_eq<T>(g, c, q);
+                if (fits) {
+                    ln.coef[C_AT][i] = q.at; ln.coef[C_AB][i] = q.ab; ln.coef[C_AN][i] = q.an; ln.coef[C_AS][i] = q.as;
+                    ln.coef[C_SU][i] = q.su; ln.coef[C_CF][i] = q.aw; ln.coef[C_PR][i] = q.ae; ln.coef[C_ID][i] = q.ap;
+                    if (fill >> D_T & 1) ln.mail[D_T][i] = q.pt;
+                    if (fill >> D_B & 1) ln.mail[D_B][i] = q.pb;
+                    if (fill >> D_N & 1) ln.mail[D_N][i] = q.pn;
+                    if (fill >> D_S & 1) ln.mail[D_S][i] = q.ps;
+                }
+            }
+            __syncwarp();
+            T *pw = fits ? ln.coef[C_CF] : g.aw + row, *pe = fits ? ln.coef[C_PR] : g.ae + row,
+              *pd = fits ? ln.coef[C_ID] : g.ap + row;
+            T *oc = fits ? ln.coef[C_CF] : g.cf + row, *op = fits ? ln.coef[C_PR] : g.pr + row,
+              *oi = fits ? ln.coef[C_ID] : g.iden + row;
+            auto get = [&](int i, T &w, T &e, T &pp) { w = pw[i]; e = pe[i]; pp = pd[i]; };
+            auto put = [&](int i, T pr, T cf, T id) { op[i] = pr; oc[i] = cf; oi[i] = id; };
+            if (!EXACT)
+                factor_line_mem<T>(n, get, put);
+            else if (lane == 0)
+                factor_line_serial<T>(n, get, put);
+            __syncwarp();
+        }
+        if (!cells) {
+            sum = cta_sum(sum, sh);
+            sumd = cta_sum(sumd, sh);
+            if (threadIdx.x == 0) {
+                double *o = red + ((size_t)(ivar - 1) * nb_region + rank) * R_NSLOTS;
+                o[ivar <= 3 ? R_MSUMD : R_MRESORM] = sum;
+                o[R_MDENOM] = sumd;
+            }
+        }
+        __syncwarp();
+        // the next equation's boundary values may change what this assembly reads
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        if (fits) {
+            // ---- the four visits of this warp's (one or two) lines ----
+            int v[2], key[2];
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                const int l = warp + s * nw;
+                v[s] = l < nloc && info[l].j >= 0 ? 0 : 4;
+            }
+            auto order = [&](int s) {
+                if (v[s] > 3) return 1 << 30;
+                const ChainInfo &f = info[warp + s * nw];
+                if (!EXACT) return 2 * v[s] + ((f.j + f.k) & 1);
+                const int m = (v[s] >> 1) * K + k1 - f.k;
+                return (3 * m + f.j - j0 + 2 * (v[s] & 1)) * 1024 + m;  // K < 512 (kChainLines x 16 lines at most)
+            };
+            key[0] = order(0);
+            key[1] = order(1);
+#pragma unroll 1
+            while (min(key[0], key[1]) < 1 << 30) {
+                const int s = key[1] < key[0] ? 1 : 0;
+                const int vs = s ? v[1] : v[0], l = warp + s * nw;
+                const ChainInfo &f = info[l];
+                ChainLine<T> &ln = lines[l];
+                const int c = (f.j + f.k) & 1;
+                const int need = chain_waits<EXACT>(vs, c, f.in), to = chain_pushes<EXACT>(vs, c, f.in);
+                if (need) {
+                    if (lane == 0)
+                        mbar_expect_tx(reinterpret_cast<uint64_t *>(&info[l].bar), (unsigned)(__popc(need) * n * sizeof(T)));
+                    __syncwarp();
+                    if (ok) ok = chain_wait(smem_u32(&f.bar), par >> s & 1, st, p.wait_polls);
+                    par ^= 1u << s;
+                }
+                T *out = vs == 3 ? phi + cidx(i0, f.j, f.k, nj, nip) : nullptr;
+                if (n <= 32)
+                    chain_visit<T, 1>(ln, f, n, to, out);
+                else
+                    chain_visit<T, 2>(ln, f, n, to, out);
+                __syncwarp();
+                if (s) {
+                    ++v[1];
+                    key[1] = order(1);
+                } else {
+                    ++v[0];
+                    key[0] = order(0);
+                }
+            }
+            __syncwarp();
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+            if (warp >= nw - idle)
+                beside(ivar, ((int)rank * idle + warp - (nw - idle)) * 32 + lane, (int)nc * idle * 32);
+        } else {
+            __syncwarp();
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+            // in place in global memory, a cluster barrier after each pass or wave
+            const int waves = EXACT ? 3 * (K - 1) + J - 1 + 2 + 1 : 2;
+            for (int sweep = 0; sweep < (EXACT ? 2 : 4); ++sweep)
+                for (int wv = 0; wv < waves; ++wv) {
+#pragma unroll 1
+                    for (int l = warp; l < nloc; l += nw) {
+                        int j, k;
+                        if (!slot_line(first + l, j, k)) continue;
+                        const int s2 = wv - 3 * (k1 - k) - (j - j0);  // exact order: 2s of a visit in this wave
+                        if (EXACT ? (s2 == 0 || s2 == 2) : ((j + k) & 1) == wv)
+                            chain_visit_mem<T>(g, phi, scratch, cidx(0, j, k, nj, nip), i0, i1, sj, sk);
+                    }
+                    cluster_barrier();
+                }
+        }
+        if (idle == 0) beside(ivar, t, nt);
+        cluster_barrier();
+    }
+    for (int q = t; q < b.n; q += nt) {
+        int i, j, k;
+        box_cell(b, q, i, j, k);
+        correct_velocity_cell<T, LD>(p, g, i, j, k);
+    }
+    if (rank == nc - 1) chain_finalize(p, st, red, cells ? nblk : (int)nc, (int)nc, nb_region, sh);
+    cluster_barrier();
+    for (int q = t; q < b.n; q += nt) {
+        int i, j, k;
+        box_cell(b, q, i, j, k);
+        correct_pressure_cell<T, LD>(p, g, i, j, k);
+    }
+}
+
 // Largest box (cells) the one-CTA / cluster path takes: one CTA's shared memory
 // holds about smem/12 cells of a thin box; a cluster of nc CTAs about nc/2 times
 // as many (slabs of whole rows, uneven by up to one row, each with two halo rows).
@@ -1711,6 +2307,43 @@ static void launch_cluster(bool pdl, void (*kern)(K...), int nc, size_t smem, cu
     cudaLaunchKernelEx(&cfg, kern, static_cast<K>(args)...);
 }
 
+// The momentum chain in one cluster launch (mom_chain_kernel): the largest cluster
+// the device schedules with its shared memory, at least 8 CTAs; chain_nc 0 where
+// there is none or it is not enabled (the serial launch form, a pinned path).
+template <typename T> int setup_mom_chain(Inst<T> &I, bool enable)
+{
+    I.chain_nc = 0;
+    if (!enable) return 0;
+    const size_t smem = chain_smem<T>();
+    void *kern = I.order == AMCFD_ORDER_EXACT ? (void *)mom_chain_kernel<T, true> : (void *)mom_chain_kernel<T, false>;
+    if (raise_smem_limit(kern, smem) != cudaSuccess ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    for (int nc : {16, 8}) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = nc;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(nc);
+        cfg.blockDim = dim3(kChainThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int m = 0;
+        if (cudaOccupancyMaxActiveClusters(&m, kern, &cfg) == cudaSuccess && m > 0) {
+            I.chain_nc = nc;
+            I.rcap = nc * kChainLines * kChainCells;
+            return 0;
+        }
+        cudaGetLastError();
+    }
+    return 0;
+}
+
 // The momentum box's red-black line solve of equation ivar as one cooperative
 // launch (mom_box_solve_kernel).
 template <typename T> static void launch_box_solve(Inst<T> &I, int ivar)
@@ -1760,6 +2393,12 @@ template <typename T> void launch_momentum(Inst<T> &I, bool small)
 {
     const int nb = I.nb_mom;
     const size_t region = (size_t)nb * R_NSLOTS;
+    if (small && I.chain_nc > 0) {
+        launch_cluster(I.pdl, I.order == AMCFD_ORDER_EXACT ? mom_chain_kernel<T, true> : mom_chain_kernel<T, false>,
+                       I.chain_nc, chain_smem<T>(), I.stream, I.p, I.g, I.red_mom, nb, I.rcell, I.rcap,
+                       I.mom_scratch);
+        return;
+    }
     if (small) {
         // assemblies over a grid sized for the box capacity (one cell a thread),
         // everything latency-bound in one CTA between them, or in one cluster of
@@ -1833,6 +2472,8 @@ template int mom_small_capacity<double>(const Inst<double> &);
 template int mom_small_capacity<float>(const Inst<float> &);
 template void setup_mom_small<double>(Inst<double> &);
 template void setup_mom_small<float>(Inst<float> &);
+template int setup_mom_chain<double>(Inst<double> &, bool);
+template int setup_mom_chain<float>(Inst<float> &, bool);
 template void setup_box_solve<double>(Inst<double> &, bool);
 template void setup_box_solve<float>(Inst<float> &, bool);
 

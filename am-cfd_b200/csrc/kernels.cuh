@@ -67,6 +67,16 @@ struct AsmMaps {
     CUtensorMap diff, h, fracl, rho, w, u, v, temp, hnot, flnot;
 };
 
+// Capacity of the one-launch momentum chain (k_momentum.cu): lines a CTA, cells a
+// line; whether a box (its extents in cells) fits a cluster of nc CTAs.
+constexpr int kChainLines = 32, kChainCells = 64;
+__host__ __device__ __forceinline__ bool chain_box_fits(int n, int nj, int nk, int exact, int nc)
+{
+    if (n <= 0 || nj <= 0 || nk <= 0) return true;  // nothing to solve
+    const long long lines = exact ? (long long)nj * nk : 2ll * ((nj + 1) / 2) * nk;
+    return n <= kChainCells && lines <= (long long)nc * kChainLines;
+}
+
 // Defect-correction buffers (AMCFD_PREC_FP32_DC, FP64 instances only): the
 // energy coefficients rounded to FP32, with `su` holding the FP64 defect
 // su + sum a_nb h_nb - ap h of the current enthalpy instead of the source; the
@@ -119,6 +129,10 @@ struct Inst {
     // multi-launch form): CTAs, warps per CTA, dynamic shared memory
     int box_grid = 0, box_warps = 4;
     size_t box_smem = 0;
+    // the momentum chain as one cluster launch (chain_nc CTAs; 0: not used), the
+    // per-cell residuals of its box (5 x rcap)
+    int chain_nc = 0, rcap = 0;
+    double *rcell = nullptr;
     // FP32 box lines' values exchanged between passes with a version tag (one
     // 64-bit word per node of the grid)
     unsigned long long *xchg = nullptr;
@@ -175,6 +189,7 @@ template <typename T> void launch_phi_sweeps(Inst<T> &I, T *phi);
 template <typename T> void launch_box_factor(Inst<T> &I);
 template <typename T> void launch_box_sweeps(Inst<T> &I, int ivar);
 template <typename T> void setup_box_solve(Inst<T> &I, bool enable);
+template <typename T> int setup_mom_chain(Inst<T> &I, bool enable);
 template <typename T> void launch_box_tickets(Inst<T> &I);
 // defect correction: the energy line sweeps in FP32 on the correction, and h += delta
 void launch_dc_sweeps(Inst<double> &I);
