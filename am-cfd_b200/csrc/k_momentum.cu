@@ -1688,7 +1688,15 @@ mom_cluster_post_kernel(Params p, Fields<T> g, T *scratch, int smem_elems, const
 //     (up to four) lines that read them, on whichever CTA of the cluster they
 //     live, by st.async: the stores complete on the receiving line's mbarrier, so
 //     a value and the news of it travel together in one hop;
-//   * launches become cluster barriers (0.2 us measured).
+//   * launches become cluster barriers, about 1 us each with the stores before
+//     them (14 of them), and the boundary values of the next equation and the
+//     residual sums run on the warps without a line while the others solve.
+// Measured (120x60x40 deck, box of 1600 cells, 98 lines on 16 CTAs): 52 us a chain
+// in FP32 and 90 in FP64, of which the eight passes take 4.2-5.6 us an equation and
+// the assembly 5.4-6.7 (FP32) and 11-15 (FP64), a serial stretch of divisions; the
+// step 4.78 -> 4.15 ms in FP32 and 6.92 -> 5.78 in FP64 (with fields read), the
+// reference's order on 61x31x21 cells 31.8 -> 18.1 ms.  L2 prefetches of the rows the
+// first assembly reads gained nothing (66.5 -> 68 us on the 400x200x100 deck).
 // The arithmetic is that of the multi-launch chain operation for operation
 // (line_rhs, the scans of solve_line_regs, factor_cell; the residual sums are
 // formed from per-cell values in the order of its per-CTA partials), so both give
@@ -1987,22 +1995,6 @@ mom_chain_kernel(Params p, Fields<T> g, double *red, int nb_region, double *rcel
         }
         f.k = k;
         mbar_init(reinterpret_cast<uint64_t *>(&f.bar));
-    }
-    // the rows the first assembly reads start towards L2 (a deck past the L2's
-    // capacity has evicted them since the iteration before), a field a lane
-    {
-        const T *src[16] = {g.uvel, g.vvel, g.wvel, g.pressure, g.vis_nxt, g.rho_nxt, g.unot, g.vnot,
-                            g.wnot, g.fracl, g.pp,  g.dux,      g.dvy,     g.dwz,     g.temp, g.temp};
-        for (int l = warp; l < nloc; l += nw) {
-            int j, k;
-            if (!slot_line(first + l, j, k)) continue;
-            const T *row = src[0];
-#pragma unroll
-            for (int a = 1; a < 16; ++a)
-                if ((lane & 15) == a) row = src[a];
-            row += cidx(lane < 16 ? i0 - 1 : i0 + n, j, k, nj, nip);
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(row));
-        }
     }
     for (int q = t; q < b.n; q += nt) {
         int i, j, k;

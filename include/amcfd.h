@@ -149,11 +149,13 @@ typedef struct amcfd_options {
     int precision;       /* AMCFD_PREC_* */
     int use_graphs;      /* capture the fixed-shape part of an outer iteration */
     int check_finite;    /* fail with AMCFD_E_NONFINITE when a reduction is not finite */
-    int no_small_box;    /* the momentum chain of a melt-pool box small enough for one CTA's
-                            shared memory (red-black order only): 0 lets the solver choose (the
-                            cooperative box solve where it is available, which measured as fast
-                            or faster for every box size, else the one-CTA chain); 1 never runs
-                            the one-CTA chain; -1 runs it whenever the box fits */
+    int no_small_box;    /* the momentum chain of a melt-pool box: 0 lets the solver choose (the
+                            whole chain in one cluster launch where the box's lines fit its
+                            shared memory, else the cooperative box solve where it is
+                            available, else, in red-black order, the one-CTA chain); 1 never
+                            runs the one-CTA chain nor the cluster launch; -1 runs the one-CTA
+                            chain whenever the box fits one CTA's shared memory (red-black
+                            order) */
     int host_loop;       /* 1: with use_graphs, still launch one graph per outer iteration and
                             test convergence on the host (0: one graph per step, the
                             iterations chained on the device) */
