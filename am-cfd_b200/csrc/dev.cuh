@@ -83,6 +83,7 @@ struct Status {
     // pipelined red-black sweep (all passes in one launch): launch sequence number,
     // CTAs done, next work ticket
     unsigned long long seq_pipe, done_pipe, ticket_pipe;
+    int bc_done;       // CTAs of the block-correction launch done with their sums
 };
 
 // Outer-loop control of a step captured as one CUDA graph (a chain of

@@ -117,30 +117,6 @@ __global__ void energy_bc_kernel(Params p, Fields<T> g, double *red)
     block_reduce_store<1>(v, s, m, red, blockIdx.x);
 }
 
-// ---------------------------------------------------------------------------
-// Block correction solve (enhanceConvergenceSpeed(5), CFDSolverManager.cpp:2334-2349)
-// and the energy residual resorh (:2099).  One CTA.
-// ---------------------------------------------------------------------------
-// Per-i sums of the block-correction partial rows in a fixed order: CTA (32 i x
-// 8 part-strides) per i-chunk and quantity.
-template <typename T>
-__global__ void __launch_bounds__(256) bc_reduce_kernel(Params p, Fields<T> g)
-{
-    pdl_enter();
-    __shared__ double sh[8][33];
-    const int i = blockIdx.x * 32 + threadIdx.x, w = blockIdx.y, nip = p.nip;
-    double s = 0.0;
-    for (int part = threadIdx.y; part < g.npart; part += 8)
-        s += g.bc[((size_t)part * 4 + w) * nip + i];
-    sh[threadIdx.y][threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.y == 0) {
-        double t = 0.0;
-        for (int y = 0; y < 8; ++y) t += sh[y][threadIdx.x];
-        g.bcsum[(size_t)w * nip + i] = t;
-    }
-}
-
 // 1-D TDMA of the block correction (enhanceConvergenceSpeed(5),
 // CFDSolverManager.cpp:2334-2349) for cells i0..i1 by one warp:
 //   den_i = bl_i - blm_i pib_{i-1},  pib_i = blp_i / den_i,
@@ -234,35 +210,78 @@ __device__ void block_tdma_warp(double *bl, double *blp, double *blm, const doub
     }
 }
 
+// ---------------------------------------------------------------------------
+// Block correction solve (enhanceConvergenceSpeed(5), CFDSolverManager.cpp:2334-2349)
+// and the energy residual resorh (:2099), in one launch.  Each CTA (32 i x 8
+// strides of the partial rows, one of the four quantities) forms its per-i sums in
+// a fixed order; the last CTA to finish solves the 1-D system with one warp while
+// the others add up the residual's per-CTA partials (32 groups of 32, the strides
+// of a 1024-thread block, then a tree over the groups).  Bound by latency: as two
+// launches 9 us on 60x30x20 cells and 20 on 400x200x100, 5 and 13 as one.
+// ---------------------------------------------------------------------------
 template <typename T>
-__global__ void block_correct_kernel(Params p, Fields<T> gd, double *red_asm, int nblk_asm,
-                                     int check_finite, int ivar)
+__global__ void __launch_bounds__(256) block_correct_kernel(Params p, Fields<T> g, const double *red_asm,
+                                                            int nblk_asm, int check_finite, int ivar)
 {
     pdl_enter();
     extern __shared__ double sm[];  // 4 * nip
+    __shared__ double sh[8][33];
+    __shared__ double grp[2][32];
+    __shared__ int last;
     const int nip = p.nip, nim2 = p.nim2;
+    {
+        const int i = blockIdx.x * 32 + threadIdx.x, w = blockIdx.y;
+        double s = 0.0;
+        const double *src = g.bc + (size_t)w * nip + i;
+#pragma unroll 8
+        for (int part = threadIdx.y; part < g.npart; part += 8) s += src[(size_t)part * 4 * nip];
+        sh[threadIdx.y][threadIdx.x] = s;
+        __syncthreads();
+        if (threadIdx.y == 0) {
+            double t = 0.0;
+            for (int y = 0; y < 8; ++y) t += sh[y][threadIdx.x];
+            g.bcsum[(size_t)w * nip + i] = t;
+            __threadfence();
+            __syncwarp();
+            if (threadIdx.x == 0) last = atomicAdd(&g.st->bc_done, 1) == (int)(gridDim.x * gridDim.y) - 1;
+        }
+        __syncthreads();
+    }
+    if (!last) return;
+    __threadfence();
+    const int tid = threadIdx.y * 32 + threadIdx.x, lane = threadIdx.x, warp = threadIdx.y;
     double *bl = sm, *blp = sm + nip, *blm = sm + 2 * nip, *blc = sm + 3 * nip;
-    for (int q = threadIdx.x; q < 4 * nip; q += blockDim.x) sm[q] = gd.bcsum[q];
-    double sd = 0.0, sh = 0.0;
-    for (int b = threadIdx.x; b < nblk_asm; b += blockDim.x) {
-        sd += red_asm[(size_t)b * R_NSLOTS + R_SUMD];
-        sh += red_asm[(size_t)b * R_NSLOTS + R_SUMH];
+    for (int q = tid; q < 4 * nip; q += 256) sm[q] = __ldcg(g.bcsum + q);
+    __syncthreads();
+    if (warp == 0) {
+        block_tdma_warp(bl, blp, blm, blc, 1, nim2, g.delphi);
+        if (lane == 0) g.st->bc_done = 0;
+    } else {
+        for (int v = warp - 1; v < 32; v += 7) {
+            double sd = 0.0, sh2 = 0.0;
+            for (int b = v * 32 + lane; b < nblk_asm; b += 1024) {
+                sd += red_asm[(size_t)b * R_NSLOTS + R_SUMD];
+                sh2 += red_asm[(size_t)b * R_NSLOTS + R_SUMH];
+            }
+            sd = warp_sum(sd);
+            sh2 = warp_sum(sh2);
+            if (lane == 0) {
+                grp[0][v] = sd;
+                grp[1][v] = sh2;
+            }
+        }
     }
     __syncthreads();
-    double v[2] = {sd, sh};
-    const int sl[2] = {0, 1};
-    const bool mx[2] = {false, false};
-    __shared__ double tot[R_NSLOTS];
-    block_reduce_store<2>(v, sl, mx, tot, 0);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        Status *st = gd.st;
-        // resorh (calculateResiduals(5)) or resorc (calculateResiduals(6))
-        double res = tot[0] / (tot[1] + kSmall);
-        if (ivar == 6) st->resorc = res; else st->resorh = res;
-        if (check_finite && !isfinite(res)) st->nonfinite = 1;
+    if (warp == 1) {
+        const double sd = warp_sum(grp[0][lane]), sh2 = warp_sum(grp[1][lane]);
+        if (lane == 0) {
+            Status *st = g.st;
+            // resorh (calculateResiduals(5)) or resorc (calculateResiduals(6))
+            const double res = sd / (sh2 + kSmall);
+            if (ivar == 6) st->resorc = res; else st->resorh = res;
+            if (check_finite && !isfinite(res)) st->nonfinite = 1;
+        }
     }
-    if (threadIdx.x < 32) block_tdma_warp(bl, blp, blm, blc, 1, nim2, gd.delphi);
 }
 // ---------------------------------------------------------------------------
 // convertEnthalpyToTemp (CFDSolverManager.cpp:2531-2571), fused with the
@@ -433,31 +452,6 @@ __global__ void __launch_bounds__(256, 4) h2t_kernel(Params p, Fields<T> g, doub
     block_reduce_store<1>(v2, s2, m2, red, blockIdx.x);
 }
 
-// Fixed-order block reduction of one slot over `nb` per-CTA partials.
-__device__ double reduce_slot(const double *red, int nb, int slot, bool is_max, double *scratch)
-{
-    double acc = is_max ? -INFINITY : 0.0;
-    for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-        double x = red[(size_t)b * R_NSLOTS + slot];
-        acc = is_max ? fmax(acc, x) : acc + x;
-    }
-    acc = is_max ? warp_max(acc) : warp_sum(acc);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) scratch[warp] = acc;
-    __syncthreads();
-    double r = is_max ? -INFINITY : 0.0;
-    if (warp == 0) {
-        r = (lane < (int)(blockDim.x >> 5)) ? scratch[lane] : (is_max ? -INFINITY : 0.0);
-        r = is_max ? warp_max(r) : warp_sum(r);
-        if (lane == 0) scratch[32] = r;
-    }
-    __syncthreads();
-    r = scratch[32];
-    __syncthreads();
-    return r;
-}
-
 // Sentinels of the melt-pool scan candidates for the next outer iteration.
 template <typename T>
 __device__ void reset_scan_candidates(const Params &p, Fields<T> &g)
@@ -479,57 +473,72 @@ __device__ void reset_scan_candidates(const Params &p, Fields<T> &g)
 // order (the NaN behaviour of std::max/min) run sequentially in thread 0.
 // Also activates the momentum box and builds its exact-order ticket list.
 // ---------------------------------------------------------------------------
-// acc = f(x_i, acc) in ascending i over the flagged i of [lo, hi), from init,
+// The reference's folds acc = f(x_i, acc) in ascending i over the flagged columns,
 // with f = std::max or std::min as the reference folds (maxd/mind): a NaN element
-// makes acc NaN and the next element replaces it.  The fold therefore equals the
+// makes acc NaN and the next element replaces it.  A fold therefore equals the
 // extreme of the flagged elements after the last NaN, NaN when that NaN is the
 // last flagged element, and includes init only when no NaN occurs -- which a
-// block can compute in two passes.  Every thread of the block calls it.
-__device__ double ordered_fold(const double *x, const int *fl, int bit, int lo, int hi, double init,
-                               bool is_max, int *si, double *sd)
+// block computes in two passes: the last flagged and the last NaN index, then
+// the extreme after it.
+__device__ __forceinline__ double fold_result(int last_flag, int last_nan, double ext, double init, bool is_max)
 {
-    const int tid = threadIdx.x, nth = blockDim.x;
-    if (tid == 0) { si[0] = -1; si[1] = -1; }
-    __syncthreads();
-    int lastf = -1, lastn = -1;  // per thread, indices ascend
-    for (int i = lo + tid; i < hi; i += nth)
-        if (fl[i] & bit) {
-            lastf = i;
-            if (isnan(x[i])) lastn = i;
-        }
-    if (lastf >= 0) atomicMax(&si[0], lastf);
-    if (lastn >= 0) atomicMax(&si[1], lastn);
-    __syncthreads();
-    const int L = si[0], P = si[1];
-    double v = is_max ? -INFINITY : INFINITY;
-    for (int i = max(lo, P + 1) + tid; i < hi; i += nth)
-        if (fl[i] & bit) v = is_max ? fmax(v, x[i]) : fmin(v, x[i]);
-    v = is_max ? warp_max(v) : -warp_max(-v);
-    if ((tid & 31) == 0) sd[tid >> 5] = v;
-    __syncthreads();
-    double r = is_max ? -INFINITY : INFINITY;
-    for (int w = 0; w < (nth + 31) / 32; ++w) r = is_max ? fmax(r, sd[w]) : fmin(r, sd[w]);
-    __syncthreads();
-    if (L < 0) return init;
-    if (P >= 0) return P == L ? (double)NAN : r;
-    return is_max ? ((r < init) ? init : r) : ((init < r) ? init : r);
+    if (last_flag < 0) return init;
+    if (last_nan >= 0) return last_nan == last_flag ? (double)NAN : ext;
+    return is_max ? ((ext < init) ? init : ext) : ((init < ext) ? init : ext);
 }
 
+// One CTA, bound by latency: a chain of block-wide reductions and gathered loads.
+// The reductions go through one shared word per warp that every warp then reduces
+// for itself (a block barrier each, four in all), and thread 0's loads for the pool
+// length are issued with the columns'.  Measured on 120x60x40 cells 17.9 -> 9 us a
+// launch (three folds of four barriers each, shared atomics from every thread).
 template <typename T>
 __global__ void __launch_bounds__(1024) meltpool_kernel(Params p, Fields<T> g, const double *red_h2t,
                                                         int nblk_h2t)
 {
     pdl_enter();
     Status *st = g.st;
-    __shared__ double scratch[40];
     extern __shared__ double colv[];  // 3 * nip doubles + nip ints
-    const int nj = p.nj, nip = p.nip;
+    __shared__ double wd[3][32];
+    __shared__ int wi[6][32];
+    const unsigned full = 0xffffffffu;
+    const int nj = p.nj, nip = p.nip, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nim1 = p.nim1, nkm1 = p.nkm1, nim2 = p.nim2, njm2 = p.njm2, nkm2 = p.nkm2;
     const double ts = p.tsolid;
-    double tp = reduce_slot(red_h2t, nblk_h2t, R_TPEAK, true, scratch);
-    double t0 = (double)g.temp[0];
+    const int js = st->jstart, is0 = st->istart, mp_imax = st->mp_imax, mp_imin = st->mp_imin;
+    const double t0 = (double)g.temp[0];
+    // peak temperature, and the column scans' candidates (gathered by h2t_kernel):
+    // depth: per column i, mp_kb = the largest k in 1..nkm2 with T < Ts on the beam
+    // plane (0 if none) -- the scan from nkm2 down visits nkm2..mp_kb+1.
+    // width: mp_jup = first j >= jstart with T < Ts (njm1 if none), mp_jdn = first
+    // j <= jstart going down with T < Ts (0 if none).
+    double tp = -INFINITY;
+    for (int b = threadIdx.x; b < nblk_h2t; b += blockDim.x)
+        tp = fmax(tp, red_h2t[(size_t)b * R_NSLOTS + R_TPEAK]);
+    int kmin_c = INT_MAX, jmax_c = INT_MIN, jmin_c = INT_MAX;
+    for (int i = 1 + (int)threadIdx.x; i < nim1; i += blockDim.x) {
+        const int kb = g.mp_kb[i], ju = g.mp_jup[i], jd = g.mp_jdn[i];
+        if (kb < nkm2) kmin_c = min(kmin_c, kb + 1);
+        if (ju > js) jmax_c = max(jmax_c, ju - 1);
+        if (jd < js) jmin_c = min(jmin_c, jd + 1);
+    }
+    tp = warp_max(tp);
+    kmin_c = __reduce_min_sync(full, kmin_c);
+    jmax_c = __reduce_max_sync(full, jmax_c);
+    jmin_c = __reduce_min_sync(full, jmin_c);
+    if (lane == 0) {
+        wd[0][warp] = tp;
+        wi[0][warp] = kmin_c; wi[1][warp] = jmax_c; wi[2][warp] = jmin_c;
+    }
+    __syncthreads();
+    tp = warp_max(wd[0][lane]);
+    kmin_c = __reduce_min_sync(full, wi[0][lane]);
+    jmax_c = __reduce_max_sync(full, wi[1][lane]);
+    jmin_c = __reduce_min_sync(full, wi[2][lane]);
     if (isnan(t0)) tp = t0;  // std::max_element keeps a leading NaN
     if (threadIdx.x == 0) st->tpeak = tp;
+    // every thread has read its candidates
+    reset_scan_candidates(p, g);
     if (!(tp > ts)) {
         if (threadIdx.x == 0) {
             st->alen = 0.0;
@@ -537,10 +546,8 @@ __global__ void __launch_bounds__(1024) meltpool_kernel(Params p, Fields<T> g, c
             st->width = 0.0;
             st->momentum_active = 0;
         }
-        reset_scan_candidates(p, g);
         return;
     }
-    const int js = st->jstart, is0 = st->istart;
     // Reads outside the node range (the reference reads past its arrays when the
     // pool touches the north/south boundary rows) return NaN instead.
     auto TT = [&](int i, int j, int k) {
@@ -551,73 +558,96 @@ __global__ void __launch_bounds__(1024) meltpool_kernel(Params p, Fields<T> g, c
     double *depv = colv, *wmax = colv + nip, *wmin = colv + 2 * nip;
     int *imaxc = (int *)(colv + 3 * nip);
     // length: first i >= istart on the top row with T <= Ts; last i <= istart with T < Ts
-    // (candidates gathered by h2t_kernel with integer atomics, read and reset here)
-    // depth: per column i, mp_kb = the largest k in 1..nkm2 with T < Ts on the beam
-    // plane (0 if none) -- the scan from nkm2 down visits nkm2..mp_kb+1.
-    // width: mp_jup = first j >= jstart with T < Ts (njm1 if none), mp_jdn = first
-    // j <= jstart going down with T < Ts (0 if none).
-    int kmin_c = INT_MAX, jmax_c = INT_MIN, jmin_c = INT_MAX;
-    for (int i = 1 + (int)threadIdx.x; i < nim1; i += blockDim.x) {
-        const int kb = g.mp_kb[i], ju = g.mp_jup[i], jd = g.mp_jdn[i];
-        if (kb < nkm2) kmin_c = min(kmin_c, kb + 1);
-        if (ju > js) jmax_c = max(jmax_c, ju - 1);
-        if (jd < js) jmin_c = min(jmin_c, jd + 1);
-    }
-    // block min/max of the integer candidates
-    __shared__ int red_i[6];
+    const int imax = (is0 < nim1) ? (mp_imax == INT_MAX ? nim1 - 1 : mp_imax) : is0;
+    const int imin = (is0 > 0) ? (mp_imin == INT_MIN ? 1 : mp_imin) : is0;
+    const int kmin = min(nkm2, kmin_c) - 1;
+    const int jmax = max(js, jmax_c) + 1;
+    const int jmin = min(js, jmin_c) - 1;
+    double xa[4], ta[4], za = 0.0, zb = 0.0;
     if (threadIdx.x == 0) {
-        red_i[0] = st->mp_imax; red_i[1] = st->mp_imin; red_i[2] = INT_MAX; red_i[3] = INT_MIN;
-        red_i[4] = INT_MAX;
+        auto XX = [&](int i) { return (i < 0 || i >= p.ni) ? (double)NAN : g.x[i]; };
+        const int at[4] = {imax, imax + 1, imin, imin - 1};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            xa[q] = XX(at[q]);
+            ta[q] = TT(at[q], js, nkm1);
+        }
+        za = g.z[nkm1];
+        zb = g.z[0];
     }
-    __syncthreads();
-    atomicMin(&red_i[2], kmin_c);
-    atomicMax(&red_i[3], jmax_c);
-    atomicMin(&red_i[4], jmin_c);
-    __syncthreads();
-    int imax = (is0 < nim1) ? (red_i[0] == INT_MAX ? nim1 - 1 : red_i[0]) : is0;
-    int imin = (is0 > 0) ? (red_i[1] == INT_MIN ? 1 : red_i[1]) : is0;
-    int kmin = min(nkm2, red_i[2]) - 1;
-    int jmax = max(js, red_i[3]) + 1;
-    int jmin = min(js, red_i[4]) - 1;
     // per-column interpolated values for the order-dependent folds
     // imaxc[i] bits: 1 = column enters the depth fold, 2 = the max-width fold,
-    // 4 = the min-width fold (the reference's `continue` tests), so that the
-    // sequential folds below read shared memory only.
+    // 4 = the min-width fold (the reference's `continue` tests); per thread, and then
+    // per block, the last flagged and the last NaN column of each fold
+    int lf[3] = {-1, -1, -1}, ln[3] = {-1, -1, -1};
     for (int i = 1 + (int)threadIdx.x; i < nim1; i += blockDim.x) {
         int fl = 0;
-        if (kmin != 0 && !(TT(i, js, kmin + 1) < ts)) {
+        const bool d0 = kmin != 0 && !(TT(i, js, kmin + 1) < ts), d1 = jmax != js && !(TT(i, jmax - 1, nkm1) < ts),
+                   d2 = jmin != js && !(TT(i, jmin + 1, nkm1) < ts);
+        if (d0) {
             fl |= 1;
             double dtdzzinv = (g.z[kmin] - g.z[kmin - 1]) / (TT(i, js, kmin) - TT(i, js, kmin - 1));
-            depv[i] = g.z[nkm1] - g.z[kmin] + (TT(i, js, kmin) - ts) * dtdzzinv;
+            const double x = g.z[nkm1] - g.z[kmin] + (TT(i, js, kmin) - ts) * dtdzzinv;
+            depv[i] = x;
+            lf[0] = i;
+            if (isnan(x)) ln[0] = i;
         }
-        if (jmax != js && !(TT(i, jmax - 1, nkm1) < ts)) {
+        if (d1) {
             fl |= 2;
             double dtdyyinv = (YY(jmax) - YY(jmax + 1)) / (TT(i, jmax, nkm1) - TT(i, jmax + 1, nkm1));
-            wmax[i] = YY(jmax) + (ts - TT(i, jmax, nkm1)) * dtdyyinv;
+            const double x = YY(jmax) + (ts - TT(i, jmax, nkm1)) * dtdyyinv;
+            wmax[i] = x;
+            lf[1] = i;
+            if (isnan(x)) ln[1] = i;
         }
-        if (jmin != js && !(TT(i, jmin + 1, nkm1) < ts)) {
+        if (d2) {
             fl |= 4;
             double dtdyyinv = (YY(jmin) - YY(jmin - 1)) / (TT(i, jmin, nkm1) - TT(i, jmin - 1, nkm1));
-            wmin[i] = YY(jmin) + (ts - TT(i, jmin, nkm1)) * dtdyyinv;
+            const double x = YY(jmin) + (ts - TT(i, jmin, nkm1)) * dtdyyinv;
+            wmin[i] = x;
+            lf[2] = i;
+            if (isnan(x)) ln[2] = i;
         }
         imaxc[i] = fl;
     }
+    __syncthreads();  // the candidates' words are read
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        lf[q] = __reduce_max_sync(full, lf[q]);
+        ln[q] = __reduce_max_sync(full, ln[q]);
+        if (lane == 0) {
+            wi[q][warp] = lf[q];
+            wi[3 + q][warp] = ln[q];
+        }
+    }
     __syncthreads();
-    // the reference's three folds over the columns (BoundCondManager.cpp:360-417),
-    // in parallel with the same NaN behaviour
-    __shared__ int fsi[2];
-    __shared__ double fsd[32];
-    const double depth_f = ordered_fold(depv, imaxc, 1, 1, nim1, 0.0, true, fsi, fsd);
-    const double ymax_f = ordered_fold(wmax, imaxc, 2, 1, nim1, g.y[0], true, fsi, fsd);
-    const double ymin_f = ordered_fold(wmin, imaxc, 4, 1, nim1, YY(js), false, fsi, fsd);
+    double ex[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        lf[q] = __reduce_max_sync(full, wi[q][lane]);
+        ln[q] = __reduce_max_sync(full, wi[3 + q][lane]);
+        ex[q] = -INFINITY;  // of the elements, or of their negatives for the minimum
+        const double *col = q == 0 ? depv : q == 1 ? wmax : wmin;
+        for (int i = 1 + (int)threadIdx.x; i < nim1; i += blockDim.x)  // this thread's own columns
+            if (i > ln[q] && (imaxc[i] >> q & 1)) ex[q] = fmax(ex[q], q == 2 ? -col[i] : col[i]);
+        ex[q] = warp_max(ex[q]);
+        if (lane == 0) wd[q][warp] = ex[q];
+    }
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) ex[q] = warp_max(wd[q][lane]);
+    }
     if (threadIdx.x == 0) {
-        auto XX = [&](int i) { return (i < 0 || i >= p.ni) ? (double)NAN : g.x[i]; };
-        double dtdxxinv = (XX(imax) - XX(imax + 1)) / (TT(imax, js, nkm1) - TT(imax + 1, js, nkm1));
-        double xxmax = XX(imax) + (ts - TT(imax, js, nkm1)) * dtdxxinv;
-        dtdxxinv = (XX(imin) - XX(imin - 1)) / (TT(imin, js, nkm1) - TT(imin - 1, js, nkm1));
-        double xxmin = XX(imin) + (ts - TT(imin, js, nkm1)) * dtdxxinv;
+        const double depth_f = fold_result(lf[0], ln[0], ex[0], 0.0, true);
+        const double ymax_f = fold_result(lf[1], ln[1], ex[1], g.y[0], true);
+        const double ymin_f = fold_result(lf[2], ln[2], -ex[2], YY(js), false);
+        double dtdxxinv = (xa[0] - xa[1]) / (ta[0] - ta[1]);
+        double xxmax = xa[0] + (ts - ta[0]) * dtdxxinv;
+        dtdxxinv = (xa[2] - xa[3]) / (ta[2] - ta[3]);
+        double xxmin = xa[2] + (ts - ta[2]) * dtdxxinv;
         st->alen = xxmax - xxmin;
-        st->depth = kmin == 0 ? g.z[nkm1] - g.z[0] : depth_f;
+        st->depth = kmin == 0 ? za - zb : depth_f;
         const double yymax = jmax != js ? ymax_f : g.y[0];
         const double yymin = jmin != js ? ymin_f : YY(js);
         st->width = yymax - yymin;
@@ -635,7 +665,6 @@ __global__ void __launch_bounds__(1024) meltpool_kernel(Params p, Fields<T> g, c
             ? max(0, st->iendm1 - st->istatp1 + 1) * max(0, st->jend - st->jstat + 1) * max(0, nkm1 - st->kstat)
             : 0;
     }
-    reset_scan_candidates(p, g);  // every reader passed the __syncthreads above
 }
 
 // ---------------------------------------------------------------------------
@@ -649,40 +678,68 @@ __global__ void converge_kernel(Params p, Fields<T> gd, const double *red_h2t, i
                                 LoopCtl lc)
 {
     pdl_enter();
-    __shared__ double scratch[40];
-    __shared__ double scr8[8 * 33];
+    // ten sums of per-CTA partials, each in the order of a one-slot block reduction
+    // (strided per-thread sums, a warp tree, a tree over the warps); a warp takes
+    // each sum's second tree, so the block meets twice instead of three times a sum
+    // (9.8 -> 6 us a launch; latency)
+    __shared__ double wsum[10][33];
     Status *st = gd.st;
-    const double *hb[8] = {red_h2t, red_h2t, red_h2t, red_h2t, red_h2t, red_h2t, red_h2t, red_h2t};
-    const int hs[8] = {R_ACCUL, R_HEATVOL, R_FW, R_FE, R_FB, R_FT, R_FS, R_FN};
-    double hv[8];
-    reduce_sums<8>(hb, hs, nb_h2t, hv, scr8);
-    const double accul = hv[0], heatvol = hv[1], fw = hv[2], fe = hv[3], fb = hv[4], ft = hv[5],
-                 fs = hv[6], fn = hv[7];
-    double ahtop = reduce_slot(red_bc, nb_bc, R_AHTOP, false, scratch);
-    double heatin = reduce_slot(red_las, nb_las, R_HEATIN, false, scratch);
+    double list[5], tpeak = 0.0, resorh = 0.0;
+    int power = 0;
     if (threadIdx.x == 0) {
+        list[0] = st->resorm; list[1] = st->resoru; list[2] = st->resorv; list[3] = st->resorw; list[4] = st->resorc;
+        tpeak = st->tpeak; resorh = st->resorh; power = st->powerindicator;
+    }
+    {
+        const int slot[10] = {R_ACCUL, R_HEATVOL, R_FW, R_FE, R_FB, R_FT, R_FS, R_FN, R_AHTOP, R_HEATIN};
+        double acc[10];
+#pragma unroll
+        for (int q = 0; q < 10; ++q) acc[q] = 0.0;
+        for (int b = threadIdx.x; b < nb_h2t; b += blockDim.x) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) acc[q] += red_h2t[(size_t)b * R_NSLOTS + slot[q]];
+        }
+        for (int b = threadIdx.x; b < nb_bc; b += blockDim.x) acc[8] += red_bc[(size_t)b * R_NSLOTS + slot[8]];
+        for (int b = threadIdx.x; b < nb_las; b += blockDim.x) acc[9] += red_las[(size_t)b * R_NSLOTS + slot[9]];
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (int)(blockDim.x >> 5);
+#pragma unroll
+        for (int q = 0; q < 10; ++q) acc[q] = warp_sum(acc[q]);
+        if (lane == 0) {
+#pragma unroll
+            for (int q = 0; q < 10; ++q) wsum[q][warp] = acc[q];
+        }
+        __syncthreads();
+        if (warp < 10) {
+            const double r = warp_sum(lane < nw ? wsum[warp][lane] : 0.0);
+            if (lane == 0) wsum[warp][32] = r;
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        const double accul = wsum[0][32], heatvol = wsum[1][32], fw = wsum[2][32], fe = wsum[3][32], fb = wsum[4][32],
+                     ft = wsum[5][32], fs = wsum[6][32], fn = wsum[7][32], ahtop = wsum[8][32], heatin = wsum[9][32];
         st->accul = p.steady ? 0.0 : accul;
         st->heatvol = p.steady ? 0.0 : heatvol;
         st->fluxwest = fw; st->fluxeast = fe; st->fluxbottom = fb; st->fluxtop = ft;
         st->fluxsouth = fs; st->fluxnorth = fn;
         st->ahtoploss = ahtop;
         st->heatinlaser = heatin;
-        st->heatout = (fn + fb + fw + fe + fs) - ahtop;
-        double ratio = p.steady ? -st->heatout / heatin : (st->heatvol + heatin) / (st->accul - st->heatout);
+        const double heatout = (fn + fb + fw + fe + fs) - ahtop;
+        st->heatout = heatout;
+        double ratio = p.steady ? -heatout / heatin : (heatvol + heatin) / (accul - heatout);
         st->ratio = ratio;
-        double list[5] = {st->resorm, st->resoru, st->resorv, st->resorw, st->resorc};
         double amaxres = list[0];
         for (int q = 1; q < 5; q++)
             if (amaxres < list[q]) amaxres = list[q];
         int conv;
         if (p.steady)
             conv = (ratio <= 1.001 && ratio >= 0.999 && amaxres < tol);
-        else if (st->powerindicator == 1)
+        else if (power == 1)
             conv = (ratio <= 1.01 && ratio >= 0.99 && amaxres < tol);
         else
-            conv = (st->resorh < 1e-6 && amaxres < tol);
+            conv = (resorh < 1e-6 && amaxres < tol);
         st->converged = conv;
-        if (check_finite && (!isfinite(st->tpeak) || !isfinite(ratio) || !isfinite(st->resorh)))
+        if (check_finite && (!isfinite(tpeak) || !isfinite(ratio) || !isfinite(resorh)))
             st->nonfinite = 1;
         if (lc.active) {
             // the host loop's bookkeeping: count the iteration, remember its box, and
@@ -763,8 +820,8 @@ template <typename T> void launch_energy_bc(Inst<T> &I)
 }
 template <typename T> void launch_block_correct(Inst<T> &I, int ivar)
 {
-    launch_k(I.pdl, bc_reduce_kernel<T>, dim3(I.p.nip / 32, 4), dim3(32, 8), 0, I.stream, I.p, I.g);
-    launch_k(I.pdl, block_correct_kernel<T>, 1, 1024, 4 * I.p.nip * sizeof(double), I.stream, I.p, I.g, I.red_asm, I.nb_asm, I.check_finite, ivar);
+    launch_k(I.pdl, block_correct_kernel<T>, dim3(I.p.nip / 32, 4), dim3(32, 8), 4 * I.p.nip * sizeof(double), I.stream,
+             I.p, I.g, I.red_asm, I.nb_asm, I.check_finite, ivar);
 }
 // Field read-out: the padded [k][j][nip] array widened to FP64 and packed to
 // the reference's unpadded [k][j][ni] layout (CFDSolverManager.cpp:249), so
