@@ -26,6 +26,7 @@ template <typename T> int exact_sweep_blocks_per_sm(int warps, size_t smem);
 template <typename T> void set_sweep_smem_limit(size_t smem);
 template <typename T> int set_rounds_smem_limit(const Params &p);
 template <typename T> int setup_pipe_sweep(const Params &p, int warps, int sm_count, size_t &smem);
+template <typename T> bool setup_resident(const Params &p);
 dim3 energy_assemble_grid(const Params &p, int kseg);
 template <typename T> int h2t_blocks_per_sm();
 template <typename T> void launch_pack_field(const T *src, double *dst, int ni, int nip,
@@ -546,6 +547,9 @@ static int setup_instance(amcfd_ctx *ctx, Inst<T> &I)
         if ((rc = alloc3<int>(ctx, &I.flags_pipe, (size_t)p.nk * p.nj))) return rc;
         I.pipe_grid = setup_pipe_sweep<T>(p, I.pipe_warps, I.sm_count, I.pipe_smem);
         if (I.dc_on) I.pipe_grid_dc = setup_pipe_sweep<float>(p, I.pipe_warps, I.sm_count, I.pipe_smem_dc);
+        // or, on a domain small enough, with every line kept by a warp
+        I.resident = (I.dc_on && !p.species) || setup_resident<T>(p);
+        if (I.dc_on) I.resident = I.resident && setup_resident<float>(p);
     }
     int bps = exact_sweep_blocks_per_sm<T>(I.exact_warps, I.line_smem);
     // A wave of the exact-order sweep holds about 2(nj-2)/3 lines; about three
@@ -1578,6 +1582,7 @@ int ctx_kind(const amcfd_ctx *ctx)
 {
     return ctx->precision + 2 * (ctx->dc ? 1 : 0) + 4 * ctx->order + 8 * (ctx->use_graphs ? 1 : 0);
 }
+bool ctx_stepped(const amcfd_ctx *ctx) { return ctx->itertot > 0; }
 double ctx_delt(const amcfd_ctx *ctx) { return ctx->delt; }
 double ctx_outtime(const amcfd_ctx *ctx) { return ctx->outtime; }
 const amcfd_params &ctx_params(const amcfd_ctx *ctx) { return ctx->prm; }

@@ -288,10 +288,17 @@ constexpr long long kSpinLimit = 1ll << 24;
 // pdl_enter: a launch's latency overlaps the run of the kernel before it instead
 // of following its drain.  Launched without the attribute, both instructions
 // return at once.
+//
+// A kernel whose CTAs run for long does the two separately: released at its start,
+// the next kernel's CTAs would hold registers and shared memory of the SMs for all
+// of that time, which kernels of other streams could use.  It waits first and releases
+// when little is left to do (a CTA that returns has released, too).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_enter()
 {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    pdl_wait();
+    pdl_release();
 }
 
 }  // namespace amcfd

@@ -78,7 +78,7 @@ template <typename T, int SCH, bool DC>
 __global__ void __launch_bounds__(256, AsmBox<T>::MINB)
 energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant__ AsmMaps mp, DcBuf dco)
 {
-    pdl_enter();
+    pdl_wait();
     using R = T;
     using B = AsmBox<T>;
     constexpr int OX = B::OX, BX = B::BX, FE = B::FE;
@@ -490,6 +490,7 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
     // per-i partial sums over this block's j-rows and planes, staged in ring A
     // (every copy has been consumed)
     double (*sb)[kTY][kTX + 1] = reinterpret_cast<double (*)[kTY][kTX + 1]>(base);
+    pdl_release();
     sb[0][ty][tx] = bl;
     sb[1][ty][tx] = blp;
     sb[2][ty][tx] = blm;

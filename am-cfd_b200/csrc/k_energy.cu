@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(256) block_correct_kernel(Params p, Fields<T> 
 template <typename T>
 __global__ void __launch_bounds__(256, 4) h2t_kernel(Params p, Fields<T> g, double *red)
 {
-    pdl_enter();
+    pdl_wait();
     const Status *st = g.st;
     const int ni = p.ni, nj = p.nj, nk = p.nk, nip = p.nip;
     const int nim1 = p.nim1, njm1 = p.njm1, nkm1 = p.nkm1, nim2 = p.nim2, njm2 = p.njm2,
@@ -408,6 +408,7 @@ __global__ void __launch_bounds__(256, 4) h2t_kernel(Params p, Fields<T> g, doub
             }
         }
     }
+    pdl_release();
     // Boundary conduction fluxes (BoundCondManager.cpp:778-843): a second pass
     // over the six interior boundary layers only, so that the bulk loop above
     // carries no flux accumulators.  Face f's layer is a 2-D index set.

@@ -316,6 +316,59 @@ __device__ __forceinline__ void ld16x(const T *ptr, T (&o)[16 / sizeof(T)])
     }
 }
 
+// The factorisation of one round of a line (V cells a lane from cell `base`): on
+// entry wc, wi, wp hold aw, ap, ae; on return cf, iden, pr (zero outside i0..i1).
+// carry_pr is pr of the cell before the round, then of its last.  The matrices
+// [[0, ae], [-aw, ap]] of the lanes below, chained by a warp scan, give a lane its
+// entry value (see factor_rounds_kernel).
+template <typename T>
+__device__ __forceinline__ void factor_round(T (&wc)[16 / sizeof(T)], T (&wi)[16 / sizeof(T)], T (&wp)[16 / sizeof(T)],
+                                             int base, int i0, int i1, T &carry_pr)
+{
+    constexpr int V = 16 / (int)sizeof(T);
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    T m00 = T(1), m01 = T(0), m10 = T(0), m11 = T(1);
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        if (base + v >= i0 && base + v <= i1) {  // [[0, ae], [-aw, ap]] * M
+            const T n00 = wp[v] * m10, n01 = wp[v] * m11;
+            const T n10 = -wc[v] * m00 + wi[v] * m10, n11 = -wc[v] * m01 + wi[v] * m11;
+            m00 = n00; m01 = n01; m10 = n10; m11 = n11;
+        }
+    }
+    mat_rescale(m00, m01, m10, m11);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const T b00 = __shfl_up_sync(full, m00, o), b01 = __shfl_up_sync(full, m01, o);
+        const T b10 = __shfl_up_sync(full, m10, o), b11 = __shfl_up_sync(full, m11, o);
+        if (lane >= o) {  // own * lower
+            const T n00 = m00 * b00 + m01 * b10, n01 = m00 * b01 + m01 * b11;
+            const T n10 = m10 * b00 + m11 * b10, n11 = m10 * b01 + m11 * b11;
+            m00 = n00; m01 = n01; m10 = n10; m11 = n11;
+            mat_rescale(m00, m01, m10, m11);
+        }
+    }
+    const T e00 = __shfl_up_sync(full, m00, 1), e01 = __shfl_up_sync(full, m01, 1);
+    const T e10 = __shfl_up_sync(full, m10, 1), e11 = __shfl_up_sync(full, m11, 1);
+    T x = carry_pr;
+    if (lane > 0) x = (e00 * carry_pr + e01) / (e10 * carry_pr + e11);
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        if (base + v >= i0 && base + v <= i1) {
+            const T den = wi[v] - wc[v] * x;
+            const T idv = T(1) / den;
+            wp[v] = wp[v] * idv;
+            wc[v] = wc[v] * idv;
+            wi[v] = idv;
+            x = wp[v];
+        } else {
+            wp[v] = wc[v] = wi[v] = T(0);
+        }
+    }
+    carry_pr = __shfl_sync(full, x, 31);
+}
+
 // One pass over the interior x-line (j, k) by the calling warp; sq/spr are the
 // warp's qr/pr buffers (2 R RC elements).  The same operations whichever kernel
 // calls it, so the per-pass launches and the pipelined launch give the same bits.
@@ -386,65 +439,30 @@ __device__ __forceinline__ void rb_line_rounds(const Params &p, const Fields<T> 
             if constexpr (FACTOR) {
                 // wc, wi, wp receive aw, ap, ae, then cf, iden, pr
                 ld16(g.aw + c, wc); ld16(g.ap + c, wi); ld16(g.ae + c, wp);
-                T m00 = T(1), m01 = T(0), m10 = T(0), m11 = T(1);
-#pragma unroll
-                for (int v = 0; v < V; ++v) {
-                    if (base + v >= i0 && base + v <= i1) {  // [[0, ae], [-aw, ap]] * M
-                        const T n00 = wp[v] * m10, n01 = wp[v] * m11;
-                        const T n10 = -wc[v] * m00 + wi[v] * m10, n11 = -wc[v] * m01 + wi[v] * m11;
-                        m00 = n00; m01 = n01; m10 = n10; m11 = n11;
-                    }
-                }
-                mat_rescale(m00, m01, m10, m11);
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const T b00 = __shfl_up_sync(full, m00, o), b01 = __shfl_up_sync(full, m01, o);
-                    const T b10 = __shfl_up_sync(full, m10, o), b11 = __shfl_up_sync(full, m11, o);
-                    if (lane >= o) {  // own * lower
-                        const T n00 = m00 * b00 + m01 * b10, n01 = m00 * b01 + m01 * b11;
-                        const T n10 = m10 * b00 + m11 * b10, n11 = m10 * b01 + m11 * b11;
-                        m00 = n00; m01 = n01; m10 = n10; m11 = n11;
-                        mat_rescale(m00, m01, m10, m11);
-                    }
-                }
-                const T e00 = __shfl_up_sync(full, m00, 1), e01 = __shfl_up_sync(full, m01, 1);
-                const T e10 = __shfl_up_sync(full, m10, 1), e11 = __shfl_up_sync(full, m11, 1);
-                T x = carry_pr;
-                if (lane > 0) x = (e00 * carry_pr + e01) / (e10 * carry_pr + e11);
-                T fpr[V], fcf[V], fid[V];
+                factor_round<T>(wc, wi, wp, base, i0, i1, carry_pr);
                 bool all = true;
 #pragma unroll
                 for (int v = 0; v < V; ++v) {
                     const bool ok = base + v >= i0 && base + v <= i1;
                     all = all && ok;
                     if (ok) {
-                        const T den = wi[v] - wc[v] * x;
-                        const T idv = T(1) / den;
-                        fpr[v] = wp[v] * idv;
-                        fcf[v] = wc[v] * idv;
-                        fid[v] = idv;
-                        x = fpr[v];
                         const T dl = (T)g.delphi[base + v];
                         if (ct) vt[v] = vt[v] + dl;
                         if (cb) vb[v] = vb[v] + dl;
                         if (cn) vn[v] = vn[v] + dl;
                         if (cs) vs[v] = vs[v] + dl;
-                    } else {
-                        fpr[v] = fcf[v] = fid[v] = T(0);
                     }
-                    wp[v] = fpr[v]; wc[v] = fcf[v]; wi[v] = fid[v];
                 }
-                carry_pr = __shfl_sync(full, x, 31);
                 if (all) {
                     typename Vec16<T>::type w;
-                    memcpy(&w, fpr, 16); *reinterpret_cast<typename Vec16<T>::type *>(g.pr + c) = w;
-                    memcpy(&w, fcf, 16); *reinterpret_cast<typename Vec16<T>::type *>(g.cf + c) = w;
-                    memcpy(&w, fid, 16); *reinterpret_cast<typename Vec16<T>::type *>(g.iden + c) = w;
+                    memcpy(&w, wp, 16); *reinterpret_cast<typename Vec16<T>::type *>(g.pr + c) = w;
+                    memcpy(&w, wc, 16); *reinterpret_cast<typename Vec16<T>::type *>(g.cf + c) = w;
+                    memcpy(&w, wi, 16); *reinterpret_cast<typename Vec16<T>::type *>(g.iden + c) = w;
                 } else if (inrow) {
 #pragma unroll
                     for (int v = 0; v < V; ++v)
                         if (base + v >= i0 && base + v <= i1) {
-                            g.pr[c + v] = fpr[v]; g.cf[c + v] = fcf[v]; g.iden[c + v] = fid[v];
+                            g.pr[c + v] = wp[v]; g.cf[c + v] = wc[v]; g.iden[c + v] = wi[v];
                         }
                 }
             } else {
@@ -627,7 +645,7 @@ __global__ void __launch_bounds__(256, 3) sweep_rb_pipe_kernel(Params p, Fields<
                                                                int *flags, unsigned long long *seqp,
                                                                unsigned long long *donep, unsigned long long *ticketp)
 {
-    pdl_enter();
+    pdl_wait();
     constexpr int RC = 32 * (16 / (int)sizeof(T));
     extern __shared__ unsigned char smraw[];
     __shared__ unsigned long long seq_s;
@@ -685,6 +703,7 @@ __global__ void __launch_bounds__(256, 3) sweep_rb_pipe_kernel(Params p, Fields<
             if (lane == 0) atomicExch(&flags[k * nj + j], base + pass + 1);
         }
     }
+    pdl_release();
     __syncthreads();
     if (threadIdx.x == 0) {
         const unsigned long long prev = atomicAdd(donep, 1ull);
@@ -695,6 +714,300 @@ __global__ void __launch_bounds__(256, 3) sweep_rb_pipe_kernel(Params p, Fields<
             __threadfence();
             atomicAdd(seqp, 1ull);
         }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The eight red-black passes of a domain small enough for every line to have a
+// warp and its coefficients a place in shared memory: one cooperative launch in
+// which a warp keeps its lines for all passes.
+//
+// What bounds such a solve is the chain of eight dependent passes, not bytes: the
+// pipelined launch spends 4.7 us a pass on a ticket, polls of four flags, loads of
+// the coefficient and neighbour rows, and two fences around the flag it sets.
+// Here a pass is: polls of four flags, the neighbours' values, two warp scans a round
+// from shared memory, and the stores.  Slots (a line of each colour, next to one
+// another in a plane) are dealt to the CTAs in plane order, one CTA a SM, a warp taking
+// every 16th slot of its CTA.  Of a line's eight rows (cf, pr, iden, formed when its
+// first pass comes, then su at ab an as) the first `nsm` stay in shared memory; the
+// others, which nothing writes, are read through L1/L2.
+// Measured (us a solve, one launch, against the pipelined form): FP32 60x30x20 26 / 35,
+// 120x60x40 32 / 38, 163x81x50 44 / 62, 200x100x60 73 / 76; FP64 131x67x41 58 / 75.
+// What is left of a pass is the way of a value and its flag between SMs: 0.85 us on one
+// die, 1.25 across (release, poll, load; a bare word takes 0.28 / 0.5).  Values that
+// carry their version in an exchange word, without flag and fence, gained 2-3 us on
+// lines of one round and lost 20-60 on longer ones, whose polls saturate the L2.
+//
+// Order.  A line's flag holds 16 x (launches so far) + passes done, set with a release
+// store after its values; a pass waits (bounded) until the flags of its four neighbours
+// show the pass before, which also says that they have read what the pass overwrites.
+// Every CTA is resident (cooperative launch) and a warp runs its lines pass by pass, so
+// every wait ends.
+//
+// The line arithmetic is rb_line_rounds' (and its factorisation's), so the results
+// are the bits of the per-pass and the pipelined launches.
+// ---------------------------------------------------------------------------
+constexpr int kResWarps = 16;
+
+// Shared memory a CTA may take, and the fewest rows worth keeping in it.
+constexpr size_t kResSmem = 224 * 1024;
+constexpr int kResMinRows = 4;
+
+enum { Q_CF = 0, Q_PR, Q_ID, Q_SU, Q_AT, Q_AB, Q_AN, Q_AS, Q_N };
+
+// Dynamic shared memory of `slots` slots (two lines each) with nsm of the eight rows.
+template <typename T> size_t resident_smem(const Params &p, int slots, int nsm)
+{
+    return (size_t)slots * 2 * nsm * p.nip * sizeof(T) + kResWarps * 8;
+}
+
+template <typename T, int R>
+__global__ void __launch_bounds__(32 * kResWarps, 1)
+sweep_resident_kernel(Params p, Fields<T> g, T *phi, int correct, int spc, int nsm, int *flags)
+{
+    pdl_wait();
+    constexpr int V = 16 / (int)sizeof(T);
+    constexpr int RC = 32 * V;
+    extern __shared__ __align__(128) unsigned char smraw[];
+    Status *st = g.st;
+    const unsigned full = 0xffffffffu;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = (int)(blockDim.x >> 5);
+    const int i0 = 1, i1 = p.nim2, j0 = 1, j1 = p.njm2, k0 = 1, k1 = p.nkm2;
+    const int nj = p.nj, nip = p.nip;
+    const size_t sj = nip, sk = (size_t)nj * nip;
+    const int half = (j1 - j0 + 2) / 2, nl = half * (k1 - k0 + 1);
+    const int first = blockIdx.x * spc, nloc = max(0, min(spc, nl - first));
+    T *sm = reinterpret_cast<T *>(smraw);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(sm + (size_t)spc * 2 * nsm * nip) + warp;
+    const int flag0 = (int)(*(volatile unsigned long long *)&st->seq_pipe * 16ull);
+    bool ok = !*(volatile int *)&st->error;
+    auto line_jk = [&](int s, int c, int &j, int &k) {
+        const int q = first + s, kk = q / half;
+        k = k0 + kk;
+        j = j0 + ((c - k - j0) % 2 + 2) % 2 + 2 * (q - kk * half);
+        return j <= j1;
+    };
+    // the vector of lane `lane` in round m: its cells, and those that are unknowns
+    unsigned okm[R];
+    int cm[R];  // first cell of the vector (the row's first vector where it lies past the row)
+#pragma unroll
+    for (int m = 0; m < R; ++m) {
+        const int base = RC * m + V * lane;
+        cm[m] = base + V <= nip ? base : 0;
+        okm[m] = 0;
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+            if (base + v >= i0 && base + v <= i1) okm[m] |= 1u << v;
+    }
+    // ---- the warp's rows into shared memory: lane r brings row r of every line ----
+    if (lane == 0) {
+        mbar_init(bar);
+        uint32_t lines = 0;
+        int j, k;
+        for (int s = warp; s < nloc; s += nw)
+            for (int c = 0; c < 2; ++c) lines += line_jk(s, c, j, k) ? 1u : 0u;
+        mbar_expect_tx(bar, lines * nsm * (uint32_t)(nip * sizeof(T)));
+    }
+    __syncwarp();
+    if (lane < nsm) {
+        const T *src = lane == Q_CF ? g.aw : lane == Q_PR ? g.ae : lane == Q_ID ? g.ap : lane == Q_SU ? g.su
+                     : lane == Q_AT ? g.at : lane == Q_AB ? g.ab : lane == Q_AN ? g.an : g.as;
+        int j, k;
+        for (int s = warp; s < nloc; s += nw)
+            for (int c = 0; c < 2; ++c)
+                if (line_jk(s, c, j, k))
+                    bulk_load(sm + ((size_t)(2 * s + c) * nsm + lane) * nip, src + cidx(0, j, k, nj, nip),
+                              (uint32_t)(nip * sizeof(T)), bar);
+    }
+    __syncwarp();
+    ok = __all_sync(full, mbar_wait(bar, 0, st, -7) && ok);
+    // ---- the passes ----
+#pragma unroll 1
+    for (int q = 0; q < 8 && ok; ++q) {
+        if (q == 6) pdl_release();
+        const int c = q & 1;
+#pragma unroll 1
+        for (int s = warp; s < nloc && ok; s += nw) {
+            int j, k;
+            if (!line_jk(s, c, j, k)) continue;
+            const size_t row = cidx(0, j, k, nj, nip);
+            T *ln = sm + (size_t)(2 * s + c) * nsm * nip;
+            const bool in[4] = {k + 1 <= k1, k - 1 >= k0, j + 1 <= j1, j - 1 >= j0};
+            const long long off[4] = {(long long)sk, -(long long)sk, (long long)sj, -(long long)sj};
+            T carry = phi[row + i0 - 1], next = phi[row + i1 + 1];
+            T a[R][V], e[R][V], A[R], B[R];
+            if (q < 2) {
+                // the line's factorisation, in place
+                T carry_pr = T(0);
+#pragma unroll
+                for (int m = 0; m < R; ++m) {
+                    T wc[V], wi[V], wp[V];
+                    ld16(ln + Q_CF * nip + cm[m], wc); ld16(ln + Q_ID * nip + cm[m], wi); ld16(ln + Q_PR * nip + cm[m], wp);
+                    factor_round<T>(wc, wi, wp, RC * m + V * lane, i0, i1, carry_pr);
+                    __syncwarp();  // a lane past the row has read the first vector
+                    if (RC * m + V * lane + V <= nip) {
+                        typename Vec16<T>::type w;
+                        memcpy(&w, wc, 16); *reinterpret_cast<typename Vec16<T>::type *>(ln + Q_CF * nip + cm[m]) = w;
+                        memcpy(&w, wi, 16); *reinterpret_cast<typename Vec16<T>::type *>(ln + Q_ID * nip + cm[m]) = w;
+                        memcpy(&w, wp, 16); *reinterpret_cast<typename Vec16<T>::type *>(ln + Q_PR * nip + cm[m]) = w;
+                    }
+                    __syncwarp();
+                }
+            }
+            if (q > 0) {
+                // lanes 0..3 poll a neighbour's flag each
+                const int dj = lane == 2 ? 1 : lane == 3 ? -1 : 0, dk = lane == 0 ? 1 : lane == 1 ? -1 : 0;
+                const bool mine = lane < 4 && k + dk >= k0 && k + dk <= k1 && j + dj >= j0 && j + dj <= j1;
+                const int *pf = flags + (k + dk) * nj + j + dj;
+                for (long long it = 0;; ++it) {
+                    int fv = 0;
+                    if (mine) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(fv) : "l"(pf) : "memory");
+                    if (__all_sync(full, !mine || fv - flag0 >= q)) break;
+                    if ((it & 63) == 63 && __any_sync(full, *(volatile int *)&st->error != 0)) ok = false;
+                    if (it > p.wait_polls) {
+                        if (lane == 0 && atomicCAS(&st->error, 0, AMCFD_E_TIMEOUT) == 0) st->error_where = k * nj + j;
+                        ok = false;
+                    }
+                    if (!ok) break;
+                }
+                if (!ok) break;
+                __syncwarp();
+            }
+            T nv[R][4][V];
+#pragma unroll
+            for (int m = 0; m < R; ++m)
+#pragma unroll
+                for (int d = 0; d < 4; ++d) {
+                    if (q == 0 && correct == 2) {
+#pragma unroll
+                        for (int v = 0; v < V; ++v) nv[m][d][v] = T(0);
+                    } else {
+                        ld16x<true>(phi + row + cm[m] + off[d], nv[m][d]);
+                    }
+                }
+            {
+#pragma unroll
+                for (int m = 0; m < R; ++m) {
+                    const int base = RC * m + V * lane;
+                    T wt[V], wb[V], wn[V], ws[V], wu[V], wc[V], wi[V];
+                    auto ldq = [&](int rw, const T *gl, T (&o)[V]) {
+                        if (rw < nsm) ld16(ln + (size_t)rw * nip + cm[m], o);
+                        else ld16(gl + row + cm[m], o);
+                    };
+                    ldq(Q_AT, g.at, wt); ldq(Q_AB, g.ab, wb); ldq(Q_AN, g.an, wn); ldq(Q_AS, g.as, ws);
+                    ldq(Q_SU, g.su, wu);
+                    ld16(ln + Q_CF * nip + cm[m], wc); ld16(ln + Q_ID * nip + cm[m], wi);
+                    T (&vt)[V] = nv[m][0], (&vb)[V] = nv[m][1], (&vn)[V] = nv[m][2], (&vs)[V] = nv[m][3];
+                    if (q == 0 && correct) {
+#pragma unroll
+                        for (int v = 0; v < V; ++v)
+                            if (okm[m] >> v & 1) {
+                                const T dl = (T)g.delphi[base + v];
+                                if (in[0]) vt[v] = vt[v] + dl;
+                                if (in[1]) vb[v] = vb[v] + dl;
+                                if (in[2]) vn[v] = vn[v] + dl;
+                                if (in[3]) vs[v] = vs[v] + dl;
+                            }
+                    }
+                    T Al = T(1), Bl = T(0);
+#pragma unroll
+                    for (int v = 0; v < V; ++v) {
+                        const bool okv = okm[m] >> v & 1;
+                        const T d = wt[v] * vt[v] + wb[v] * vb[v] + wn[v] * vn[v] + ws[v] * vs[v] + wu[v];
+                        a[m][v] = okv ? wc[v] : T(1);
+                        e[m][v] = okv ? d * wi[v] : T(0);
+                        Bl = a[m][v] * Bl + e[m][v];
+                        Al = a[m][v] * Al;
+                    }
+                    A[m] = Al;
+                    B[m] = Bl;
+                }
+            }
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+                for (int m = 0; m < R; ++m) {
+                    const T A2 = __shfl_up_sync(full, A[m], o), B2 = __shfl_up_sync(full, B[m], o);
+                    if (lane >= o) {
+                        B[m] = A[m] * B2 + B[m];
+                        A[m] = A[m] * A2;
+                    }
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < R; ++m) {
+                T Ae = __shfl_up_sync(full, A[m], 1), Be = __shfl_up_sync(full, B[m], 1);
+                if (lane == 0) { Ae = T(1); Be = T(0); }
+                T x = Ae * carry + Be;
+#pragma unroll
+                for (int v = 0; v < V; ++v) {
+                    x = a[m][v] * x + e[m][v];
+                    e[m][v] = x;  // qr
+                }
+                carry = __shfl_sync(full, A[m] * carry + B[m], 31);
+            }
+            // backward: a holds pr
+#pragma unroll
+            for (int m = 0; m < R; ++m) {
+                T wp[V];
+                ld16(ln + Q_PR * nip + cm[m], wp);
+                T Al = T(1), Bl = T(0);
+#pragma unroll
+                for (int v = V - 1; v >= 0; --v) {
+                    const bool okv = okm[m] >> v & 1;
+                    e[m][v] = okv ? e[m][v] : T(0);
+                    a[m][v] = okv ? wp[v] : T(1);
+                    Bl = a[m][v] * Bl + e[m][v];
+                    Al = a[m][v] * Al;
+                }
+                A[m] = Al;
+                B[m] = Bl;
+            }
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+                for (int m = 0; m < R; ++m) {
+                    const T A2 = __shfl_down_sync(full, A[m], o), B2 = __shfl_down_sync(full, B[m], o);
+                    if (lane + o < 32) {
+                        B[m] = A[m] * B2 + B[m];
+                        A[m] = A[m] * A2;
+                    }
+                }
+            }
+#pragma unroll
+            for (int m = R - 1; m >= 0; --m) {
+                T Ae = __shfl_down_sync(full, A[m], 1), Be = __shfl_down_sync(full, B[m], 1);
+                if (lane == 31) { Ae = T(1); Be = T(0); }
+                T x = Ae * next + Be;
+                T out[V];
+#pragma unroll
+                for (int v = V - 1; v >= 0; --v) {
+                    x = a[m][v] * x + e[m][v];
+                    out[v] = x;
+                }
+                if (okm[m] == (1u << V) - 1u) {
+                    typename Vec16<T>::type w;
+                    memcpy(&w, out, 16);
+                    *reinterpret_cast<typename Vec16<T>::type *>(phi + row + cm[m]) = w;
+                } else {
+#pragma unroll
+                    for (int v = 0; v < V; ++v)
+                        if (okm[m] >> v & 1) phi[row + cm[m] + v] = out[v];
+                }
+                next = __shfl_sync(full, A[m] * next + B[m], 0);
+            }
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(flags + k * nj + j), "r"(flag0 + q + 1) : "memory");
+        }
+    }
+    // the last CTA through advances the launch count (the pipelined launch's, whose
+    // flags these are)
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&st->done_pipe, 1ull) == (unsigned long long)gridDim.x - 1) {
+        atomicExch(&st->done_pipe, 0ull);
+        __threadfence();
+        atomicAdd(&st->seq_pipe, 1ull);
     }
 }
 
@@ -893,6 +1206,55 @@ template <typename T> void launch_box_factor(Inst<T> &I)
     int grid = std::min((I.max_lines + 31) / 32, I.sm_count);
     launch_k(I.pdl, factor_kernel<T, true>, grid, 256, 0, I.stream, I.p, I.g, nullptr);
 }
+// Launch shape of the resident sweep on the active domain: rounds a line, slots a
+// CTA (one CTA a SM) and coefficient rows kept in shared memory; false where the
+// lines are too long or too many for it.
+template <typename S> static bool resident_shape(const Params &p, int sm_count, int &R, int &spc, int &nsm)
+{
+    const int RC = 32 * (16 / (int)sizeof(S));
+    const int nl = ((p.nj - 2 + 1) / 2) * (p.nk - 2);
+    if (nl <= 0 || p.nim2 < 1) return false;
+    R = p.nim2 / RC + 1;
+    spc = (nl + sm_count - 1) / sm_count;
+    if (R > 4) return false;
+    for (nsm = Q_N; nsm >= kResMinRows; --nsm)
+        if (resident_smem<S>(p, spc, nsm) <= kResSmem) return true;
+    return false;
+}
+template <typename S> static auto resident_kernel(int R)
+{
+    return R == 1 ? sweep_resident_kernel<S, 1> : R == 2 ? sweep_resident_kernel<S, 2>
+         : R == 3 ? sweep_resident_kernel<S, 3> : sweep_resident_kernel<S, 4>;
+}
+template <typename T, typename S> static bool launch_resident(Inst<T> &I, const Fields<S> &g, S *phi, int correct)
+{
+    int R, spc, nsm;
+    if (!I.resident || !resident_shape<S>(I.p, I.sm_count, R, spc, nsm)) return false;
+    const int nl = ((I.p.nj - 2 + 1) / 2) * (I.p.nk - 2);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.gridDim = dim3((nl + spc - 1) / spc);
+    cfg.blockDim = dim3(32 * std::min(kResWarps, spc));  // (other streams' kernels share the SMs)
+    cfg.dynamicSmemBytes = resident_smem<S>(I.p, spc, nsm);
+    cfg.stream = I.stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, resident_kernel<S>(R), I.p, g, phi, correct, spc, nsm, I.flags_pipe);
+    return true;
+}
+// Raises the shared-memory limit of the resident sweep's kernels (whichever line
+// length the domain has); false where that fails.
+template <typename S> bool setup_resident(const Params &p)
+{
+    int R, spc, nsm;
+    if (!resident_shape<S>(p, 1 << 20, R, spc, nsm)) return false;
+    if (raise_smem_limit((const void *)resident_kernel<S>(R), kResSmem) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+
 template <typename T> static void sweeps(Inst<T> &I, T *phi, bool box)
 {
     const int warps = I.exact_warps;
@@ -912,6 +1274,8 @@ template <typename T> static void sweeps(Inst<T> &I, T *phi, bool box)
         for (int sweep = 0; sweep < 4; ++sweep)
             for (int color = 0; color < 2; ++color)
                 launch_k(I.pdl, sweep_rb_kernel<T, true>, grid, 32 * warps, smem, I.stream, I.p, I.g, phi, color);
+    } else if (launch_resident<T, T>(I, I.g, phi, 1)) {
+        // whole domain, every line kept by a warp for the eight passes
     } else if (I.pipe_grid > 0) {
         // whole domain, the eight passes in one pipelined launch
         Status *st = I.g.st;
@@ -961,6 +1325,7 @@ void launch_dc_sweeps(Inst<double> &I)
     f.pr = d.pr; f.cf = d.cf; f.iden = d.iden;
     f.delphi = I.g.delphi;
     f.st = I.g.st;
+    if (launch_resident<double, float>(I, f, d.delta, 2)) return;
     if (I.pipe_grid_dc > 0) {
         Status *st = I.g.st;
         launch_k(I.pdl, sweep_rb_pipe_kernel<float>, I.pipe_grid_dc, 32 * I.pipe_warps, I.pipe_smem_dc, I.stream, I.p,
@@ -1076,6 +1441,7 @@ template <typename T> int setup_pipe_sweep(const Params &p, int warps, int sm_co
 
 #define AMCFD_INST(T)                                                     \
     template int setup_pipe_sweep<T>(const Params &, int, int, size_t &); \
+    template bool setup_resident<T>(const Params &);                      \
     template void launch_energy_factor<T>(Inst<T> &);                    \
     template void launch_box_factor<T>(Inst<T> &);                       \
     template void launch_energy_sweeps<T>(Inst<T> &);                    \

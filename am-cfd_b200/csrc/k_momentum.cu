@@ -1937,7 +1937,7 @@ template <typename T, bool EXACT>
 __global__ void __launch_bounds__(kChainThreads, 1)
 mom_chain_kernel(Params p, Fields<T> g, double *red, int nb_region, double *rcell, int rcap, T *scratch)
 {
-    pdl_enter();
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ double sh[40];
     ChainLine<T> *lines = reinterpret_cast<ChainLine<T> *>(smraw);
@@ -2054,6 +2054,7 @@ mom_chain_kernel(Params p, Fields<T> g, double *red, int nb_region, double *rcel
     const int idle = fits && lpc < nw ? nw - lpc : 0;
 #pragma unroll 1
     for (int ivar = 1; ivar <= 4; ++ivar) {
+        if (ivar == 4) pdl_release();
         T *phi = ivar == 1 ? g.uvel : ivar == 2 ? g.vvel : ivar == 3 ? g.wvel : g.pp;
         // ---- assembly and factorisation of this warp's lines ----
         double sum = 0.0, sumd = 0.0;

@@ -145,6 +145,8 @@ struct Inst {
     int pipe_grid = 0, pipe_warps = 8, pipe_grid_dc = 0, pipe_stride = 16;
     size_t pipe_smem = 0, pipe_smem_dc = 0;
     int *flags_pipe = nullptr;
+    // or, on a domain small enough (checked at each launch), with every line kept by a warp
+    bool resident = false;
 };
 
 // Launch of a kernel that begins with pdl_enter().  With `pdl` the launch carries
