@@ -298,7 +298,10 @@ static int alloc3(amcfd_ctx *ctx, T **ptr, size_t n)
         return AMCFD_E_NOMEM;
     }
     ctx->allocs.push_back(p);
-    cudaMemsetAsync(p, 0, n * sizeof(T), ctx->stream);
+    // on the legacy stream, like the copies that fill some of these arrays next: the
+    // context's own stream does not order with it, and a late memset there would
+    // clear what they brought
+    cudaMemset(p, 0, n * sizeof(T));
     *ptr = (T *)p;
     return 0;
 }
@@ -349,6 +352,7 @@ static int set_active_nk(amcfd_ctx *ctx, Inst<T> &I, int nk)
     I.max_lines = (p.nj - 2) * (p.nk - 2);
     const std::vector<int2> tk = energy_tickets(p.nk - 2, p.nj - 2);
     CK(cudaMemcpy(I.g.tickets_energy, tk.data(), tk.size() * sizeof(int2), cudaMemcpyHostToDevice));
+    CK(cudaStreamSynchronize(cudaStreamLegacy));
     I.g.ntickets_energy = (int)tk.size();
     drop_graphs(ctx);
     return 0;
@@ -610,7 +614,7 @@ static int setup_instance(amcfd_ctx *ctx, Inst<T> &I)
     for (int k = 0; k < p.nk; k++)
         for (int i = 0; i < p.ni; i++) hv[cidx(i, p.njm1, k, p.nj, p.nip)] = enth(q.tempnorth);
     if ((rc = upload<T>(ctx, g.h, hv))) return rc;
-    CK(cudaStreamSynchronize(ctx->stream));
+    CK(cudaStreamSynchronize(cudaStreamLegacy));  // before the context's stream reads any of it
     // powder bed: only the first layer starts active (PrintManager.cpp:67-73)
     return set_active_nk<T>(ctx, I, ctx->nk_active);
 }
@@ -1643,7 +1647,7 @@ int amcfd_ws_attach(amcfd_ctx *ctx, amcfd_net *net, int mode)
     CK(cudaMalloc(&ctx->ws_feat, n * 11 * sizeof(float)));
     CK(cudaMalloc(&ctx->ws_y, n * 2 * sizeof(float)));
     CK(cudaMalloc(&ctx->ws_target, n * 2 * sizeof(float)));
-    CK(cudaMemset(ctx->ws_target, 0, n * 2 * sizeof(float)));
+    CK(cudaMemsetAsync(ctx->ws_target, 0, n * 2 * sizeof(float), ctx->stream));
     for (auto &q : ctx->ws_save) CK(cudaMalloc(&q, n3 * e));
     return 0;
 }
@@ -1874,6 +1878,7 @@ int amcfd_set_field(amcfd_ctx *ctx, const char *name, const double *host_in)
         CK(cudaMemcpy2D(d, ctx->nip * sizeof(float), tmp.data(), ctx->ni * sizeof(float),
                         ctx->ni * sizeof(float), rows, cudaMemcpyHostToDevice));
     }
+    CK(cudaStreamSynchronize(cudaStreamLegacy));  // the context's stream does not order with the copy
     return 0;
 }
 
