@@ -22,6 +22,7 @@
 // properties and divisions in FP32, and it and the defect-correction build form
 // each face's conductance and Peclet number from one reciprocal.
 #include <algorithm>
+#include <type_traits>
 
 #include "kernels.cuh"
 #include "async.cuh"
@@ -43,9 +44,6 @@ template <typename T> struct AsmBox {
     static constexpr int NA = 5, NB = 5, SA = 4, SB = 2;
     // rings + mbarriers + slack to align the dynamic region to 128 bytes
     static constexpr size_t SMEM = (size_t)(SA * NA + SB * NB) * FE * sizeof(T) + 8 * (SA + SB) + 128;
-    // resident CTAs per SM: three in FP32 (80 registers a thread still hold the
-    // whole stencil), two in FP64
-    static constexpr int MINB = sizeof(T) == 4 ? 3 : 2;
 };
 // Warps of a CTA, and the plane-completion counters (a warp is at most one
 // plane ahead of the slowest, so four counters never mix two planes).
@@ -58,15 +56,48 @@ enum { FB_U = 0, FB_V, FB_T, FB_HN, FB_FN };
 // one reciprocal r = 1 / (num den): d = num^2 r and |F| / d = |F| den^2 r.
 __device__ __forceinline__ float rcp_fast(float x) { return __fdividef(1.0f, x); }
 __device__ __forceinline__ double rcp_fast(double x) { return 1.0 / x; }
-template <typename R>
+// a b + c with one rounding, whichever of a sum's two products the compiler would fuse.
+__device__ __forceinline__ float fused(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fused(double a, double b, double c) { return __fma_rn(a, b, c); }
+// A product as its own rounded value: the sums it enters must not fuse with it, as they
+// do not with the long form's coefficient.
+__device__ __forceinline__ float rounded(float x)
+{
+    asm("" : "+f"(x));
+    return x;
+}
+__device__ __forceinline__ double rounded(double x)
+{
+    asm("" : "+d"(x));
+    return x;
+}
+template <typename R, bool STILL>
 __device__ __forceinline__ void face_fast(int sch, R num, R den, R f, R &plus, R &minus)
 {
     const R r = rcp_fast(num * den);
     const R d = num * num * r;
-    const R a = d * scheme_fn<R>(sch, fabs(f) * (den * den * r));
-    plus = a + maxd(R(0), -f);
-    minus = a + maxd(R(0), f);
+    if constexpr (STILL) {
+        plus = minus = rounded(d);
+    } else {
+        const R a = d * scheme_fn<R>(sch, fabs(f) * (den * den * r));
+        plus = a + maxd(R(0), -f);
+        minus = a + maxd(R(0), f);
+    }
 }
+// The reference's form (face_coef); without a mass flux, the conductance alone.
+template <typename R, bool STILL>
+__device__ __forceinline__ void face_ref(int sch, R d, R f, R &plus, R &minus)
+{
+    if constexpr (STILL)
+        plus = minus = rounded(d);
+    else
+        face_coef<R>(sch, d, f, plus, minus);
+}
+
+// Per-launch constants of the assembly, rounded to the bulk precision.
+template <typename R> struct AsmConst {
+    R thla, thlb, acpl, thsa, thsb, thsc, acpa, acpb, tliq, tsol, denl, dens, visc, urfh, hlatnt, inv_acpl, inv_urfh;
+};
 
 // SCH: the discretisation scheme as a compile-time constant (one instantiation per
 // scheme), so that the six face coefficients carry no untaken scheme branches.
@@ -74,9 +105,22 @@ __device__ __forceinline__ void face_fast(int sch, R num, R den, R f, R &plus, R
 // the fast builds' one reciprocal per face), stored rounded to FP32 in `dco`, and
 // the FP32 `su` slot receives the FP64 defect su + sum a_nb h_nb - ap h of the
 // current enthalpy; the FP64 coefficient arrays are not written.
-template <typename T, int SCH, bool DC>
-__global__ void __launch_bounds__(256, AsmBox<T>::MINB)
-energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant__ AsmMaps mp, DcBuf dco)
+//
+// CALM: warps whose cells see no flow take the short form of a cell (STILL below), with
+// OCC resident CTAs a SM.  Nearly all warps of a deck do: a melt pool is a few thousand
+// cells.  The long form is bound by issue (659 instructions a warp and plane in FP32, XU
+// 30 %) and in FP64 by its divisions.  Measured (us a launch with its boundary and
+// block-correction kernels): 400x200x100 FP32 230 -> 208, DC 380 -> 330, FP64 588 -> 349;
+// 600x300x120 FP32 536 -> 473; 120x60x40 FP32 34.5 -> 31.  On a grid of at most one CTA a
+// SM (60x30x20) a CTA's own latency counts, and fetching two forms' instructions costs
+// more than the short one saves (26.7 -> 28.6): those run without.  Four CTAs a SM in
+// FP32 (64 registers, some spilled in the long form) hide more of the planes' latency
+// where there are CTAs for them (225 -> 208 on 400x200x100) and cost the spills where
+// there are not (32.7 -> 36.5 on 120x60x40).
+template <typename T, int SCH, bool DC, bool CALM, int OCC>
+__global__ void __launch_bounds__(256, OCC)
+energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant__ AsmMaps mp, DcBuf dco,
+                       const __grid_constant__ AsmConst<T> cst)
 {
     pdl_wait();
     using R = T;
@@ -96,8 +140,7 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
     const int i = blockIdx.x * kTX + tx, j = blockIdx.y * kTY + ty;
     const int x0 = blockIdx.x * kTX - OX, y0 = blockIdx.y * kTY - 1;
     const int ni = p.ni, nj = p.nj, nk = p.nk, nip = p.nip;
-    const int nim1 = p.nim1, njm1 = p.njm1, nkm1 = p.nkm1, nim2 = p.nim2, njm2 = p.njm2,
-              nkm2 = p.nkm2;
+    const int nkm1 = p.nkm1, nim2 = p.nim2, njm2 = p.njm2, nkm2 = p.nkm2;
     const int kseg = (nk + gridDim.z - 1) / gridDim.z;
     const int kb = blockIdx.z * kseg, ke = min(kb + kseg, nk);
     const bool in = (i < ni && j < nj);
@@ -192,14 +235,12 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
     // and the divisions by per-launch constants as multiplications
     constexpr bool FAST = kF32 || DC;
     const R fdx = (R)dx, fdy = (R)dy;
-    const R inv_acpl = (R)(1.0 / p.acpl), inv_delt = (R)(1.0 / delt), inv_urfh = (R)(1.0 / p.urfh);
-    const R dxp_e = (R)g.dxpwinv[nim1], dxp_w = (R)g.dxpwinv[1];
-    const R dyp_n = (R)g.dypsinv[njm1], dyp_s = (R)g.dypsinv[1];
-    const R dzp_t = (R)g.dzpbinv[nkm1], dzp_b = (R)g.dzpbinv[1];
-    const R thla = (R)p.thconla, thlb = (R)p.thconlb, acpl = (R)p.acpl, thsa = (R)p.thconsa,
-            thsb = (R)p.thconsb, thsc = (R)p.thconsc, acpa = (R)p.acpa, acpb = (R)p.acpb,
-            tliq = (R)p.tliquid, tsol = (R)p.tsolid, denl = (R)p.denl, dens = (R)p.dens,
-            visc = (R)p.viscos;
+    const R inv_delt = (R)(1.0 / delt);
+    // per-launch constants in the bulk precision stay in the kernel's parameters (as
+    // registers they cost the FP32 build a quarter of its budget)
+    const R &inv_acpl = cst.inv_acpl, &inv_urfh = cst.inv_urfh, &thla = cst.thla, &thlb = cst.thlb, &acpl = cst.acpl,
+            &thsa = cst.thsa, &thsb = cst.thsb, &thsc = cst.thsc, &acpa = cst.acpa, &acpb = cst.acpb,
+            &tliq = cst.tliq, &tsol = cst.tsol, &denl = cst.denl, &dens = cst.dens, &visc = cst.visc;
     double sumd = 0.0, sumh = 0.0;
     double bl = 0.0, blp = 0.0, blm = 0.0, blc = 0.0;
     const int o = (ty + 1) * BX + tx + OX;  // this thread's cell inside a box
@@ -217,6 +258,10 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
         const T *Ap = bufA + slotA(k + 1) * B::NA * FE + o;  // plane k+1
         const T *Bc = bufB + slotB(k) * B::NB * FE + o;      // plane k
         const size_t c = col + (size_t)k * sk;
+        const bool cell = colint && k >= 1 && k <= nkm2;
+        const bool still = CALM && SCH != 2 && __all_sync(0xffffffffu, !cell || (Bc[FB_U * FE] == R(0) && Bc[FB_U * FE + 1] == R(0) &&
+                                                                         Bc[FB_V * FE] == R(0) && Bc[FB_V * FE + BX] == R(0) &&
+                                                                         Ac[FA_W * FE] == R(0) && Ap[FA_W * FE] == R(0)));
         if (in) {
             const R d_c = Ac[FA_D * FE], f_c = Ac[FA_F * FE], t_c = Bc[FB_T * FE];
             // ---- material properties (every node) ----
@@ -242,7 +287,7 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
                     dn = diffs; rn = rs; vn = R(1e10);
                     if (!(t <= tsol)) {
                         dn = fl * diffl + (R(1) - fl) * diffs;
-                        rn = fl * denl + (R(1) - fl) * rs;
+                        rn = fused(fl, denl, (R(1) - fl) * rs);
                         vn = visc;
                     }
                 }
@@ -250,7 +295,12 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
                 g.rho_nxt[c] = rn;
                 g.vis_nxt[c] = vn;
             }
-            if (colint && k >= 1 && k <= nkm2) {
+            // One interior cell.  STILL: the six face velocities of every interior cell of the
+            // warp are zero, so no face carries a mass flux: each coefficient is the face's
+            // conductance (the scheme's A(0) = 1 exactly) and the convected latent heat is
+            // nothing -- the same numbers without forming them.
+            auto interior = [&](auto still_c) {
+                constexpr bool STILL = decltype(still_c)::value;
                 const int kl = k - kb;
                 const double dz = pl_dz[kl];
                 const R fdz = pl_m[4][kl];
@@ -267,97 +317,97 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
                 const R w_c = Ac[FA_W * FE], w_p = Ap[FA_W * FE];
                 // north face
                 {
-                    R fn = Ac[FA_R * FE + BX] * v_n * aik;
+                    const R fn = STILL ? R(0) : Ac[FA_R * FE + BX] * v_n * aik;
                     if constexpr (FAST) {
                         const bool bnd = j == njm2;
-                        const R num = bnd ? dcc * aik * dyp_n : dcc * d_nn * aik * dyp_p;
+                        const R num = bnd ? dcc * aik * dyp_p : dcc * d_nn * aik * dyp_p;
                         const R den = bnd ? R(1) : (R(1) - fy_j) * d_nn + fy_j * dcc;
-                        face_fast<R>(sch, num, den, fn, an, tmp);
+                        face_fast<R, STILL>(sch, num, den, fn, an, tmp);
                     } else {
                         R dn;
                         if (j == njm2) {
-                            dn = dcc * aik * dyp_n;
+                            dn = dcc * aik * dyp_p;
                         } else {
                             R difn = bdiv(dcc * d_nn, (R(1) - fy_j) * d_nn + fy_j * dcc);
                             dn = difn * aik * dyp_p;
                         }
-                        face_coef<R>(sch, dn, fn, an, tmp);
+                        face_ref<R, STILL>(sch, dn, fn, an, tmp);
                     }
                 }
                 // south face
                 {
-                    R fs = rhc * v_c * aik;
+                    const R fs = STILL ? R(0) : rhc * v_c * aik;
                     if constexpr (FAST) {
                         const bool bnd = j == 1;
-                        const R num = bnd ? dcc * aik * dyp_s : d_s * dcc * aik * dyp_j;
+                        const R num = bnd ? dcc * aik * dyp_j : d_s * dcc * aik * dyp_j;
                         const R den = bnd ? R(1) : (R(1) - fy_m) * dcc + fy_m * d_s;
-                        face_fast<R>(sch, num, den, fs, tmp, as_);
+                        face_fast<R, STILL>(sch, num, den, fs, tmp, as_);
                     } else {
                         R ds;
                         if (j == 1) {
-                            ds = dcc * aik * dyp_s;
+                            ds = dcc * aik * dyp_j;
                         } else {
                             R difs = bdiv(d_s * dcc, (R(1) - fy_m) * dcc + fy_m * d_s);
                             ds = difs * aik * dyp_j;
                         }
-                        face_coef<R>(sch, ds, fs, tmp, as_);
+                        face_ref<R, STILL>(sch, ds, fs, tmp, as_);
                     }
                 }
                 // east face
                 {
-                    R fe = Ac[FA_R * FE + 1] * u_e * ajk;
+                    const R fe = STILL ? R(0) : Ac[FA_R * FE + 1] * u_e * ajk;
                     if constexpr (FAST) {
                         const bool bnd = i == nim2;
-                        const R num = bnd ? dcc * ajk * dxp_e : dcc * d_e * ajk * dxp_p;
+                        const R num = bnd ? dcc * ajk * dxp_p : dcc * d_e * ajk * dxp_p;
                         const R den = bnd ? R(1) : (R(1) - fx_i) * d_e + fx_i * dcc;
-                        face_fast<R>(sch, num, den, fe, ae, tmp);
+                        face_fast<R, STILL>(sch, num, den, fe, ae, tmp);
                     } else {
                         R de;
                         if (i == nim2) {
-                            de = dcc * ajk * dxp_e;
+                            de = dcc * ajk * dxp_p;
                         } else {
                             R dife = bdiv(dcc * d_e, (R(1) - fx_i) * d_e + fx_i * dcc);
                             de = dife * ajk * dxp_p;
                         }
-                        face_coef<R>(sch, de, fe, ae, tmp);
+                        face_ref<R, STILL>(sch, de, fe, ae, tmp);
                     }
                 }
                 // west face
                 {
-                    R fw = rhc * u_c * ajk;
+                    const R fw = STILL ? R(0) : rhc * u_c * ajk;
                     if constexpr (FAST) {
                         const bool bnd = i == 1;
-                        const R num = bnd ? dcc * ajk * dxp_w : d_w * dcc * ajk * dxp_i;
+                        const R num = bnd ? dcc * ajk * dxp_i : d_w * dcc * ajk * dxp_i;
                         const R den = bnd ? R(1) : (R(1) - fx_m) * dcc + fx_m * d_w;
-                        face_fast<R>(sch, num, den, fw, tmp, aw);
+                        face_fast<R, STILL>(sch, num, den, fw, tmp, aw);
                     } else {
                         R dw;
                         if (i == 1) {
-                            dw = dcc * ajk * dxp_w;
+                            dw = dcc * ajk * dxp_i;
                         } else {
                             R difw = bdiv(d_w * dcc, (R(1) - fx_m) * dcc + fx_m * d_w);
                             dw = difw * ajk * dxp_i;
                         }
-                        face_coef<R>(sch, dw, fw, tmp, aw);
+                        face_ref<R, STILL>(sch, dw, fw, tmp, aw);
                     }
                 }
                 // top face
                 {
-                    R ft = Ap[FA_R * FE] * w_p * aij;
+                    const R ft = STILL ? R(0) : Ap[FA_R * FE] * w_p * aij;
                     if constexpr (FAST) {
                         const bool bnd = k == nkm2;
-                        const R num = bnd ? dcc * aij * dzp_t : dcc * d_p * aij * dzp_p;
+                        const R num = bnd ? dcc * aij * dzp_p : dcc * d_p * aij * dzp_p;
                         const R den = bnd ? R(1) : (R(1) - fz_k) * d_p + fz_k * dcc;
-                        face_fast<R>(sch, num, den, ft, at, ab_up);
+                        face_fast<R, STILL>(sch, num, den, ft, at, ab_up);
                     } else {
                         R dt;
                         if (k == nkm2) {
-                            dt = dcc * aij * dzp_t;
+                            dt = dcc * aij * dzp_p;
                         } else {
                             R dift = bdiv(dcc * d_p, (R(1) - fz_k) * d_p + fz_k * dcc);
                             dt = dift * aij * dzp_p;
                         }
-                        face_coef<R>(sch, dt, ft, at, ab_up);
+                        face_ref<R, STILL>(sch, dt, ft, at, ab_up);
                     }
                 }
                 // bottom face: the top face of the plane below, as this thread formed
@@ -366,21 +416,21 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
                 if (k > kb && k > 1) {
                     ab = ab_bottom;
                 } else {
-                    R fb = rhc * w_c * aij;
+                    const R fb = STILL ? R(0) : rhc * w_c * aij;
                     if constexpr (FAST) {
                         const bool bnd = k == 1;
-                        const R num = bnd ? dcc * aij * dzp_b : d_m * dcc * aij * dzp_k;
+                        const R num = bnd ? dcc * aij * dzp_k : d_m * dcc * aij * dzp_k;
                         const R den = bnd ? R(1) : (R(1) - fz_m) * dcc + fz_m * d_m;
-                        face_fast<R>(sch, num, den, fb, tmp, ab);
+                        face_fast<R, STILL>(sch, num, den, fb, tmp, ab);
                     } else {
                         R db;
                         if (k == 1) {
-                            db = dcc * aij * dzp_b;
+                            db = dcc * aij * dzp_k;
                         } else {
                             R difb = bdiv(d_m * dcc, (R(1) - fz_m) * dcc + fz_m * d_m);
                             db = difb * aij * dzp_k;
                         }
-                        face_coef<R>(sch, db, fb, tmp, ab);
+                        face_ref<R, STILL>(sch, db, fb, tmp, ab);
                     }
                 }
                 ab_bottom = ab_up;
@@ -401,12 +451,12 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
                     }
                     g.sourceinput[c] = srcin;
                 }
-                const R hlatnt = (R)p.hlatnt;
+                const R hlatnt = cst.hlatnt;
                 const R variable1 = FAST ? hlatnt * rhc * inv_delt : bdiv(hlatnt * rhc, (R)delt);
                 const R volht = vol * variable1;
                 const R flc = f_c;
                 su -= volht * (flc - Bc[FB_FN * FE]);
-                {
+                if constexpr (!STILL) {
                     const R fl_w = Ac[FA_F * FE - 1], fl_e = Ac[FA_F * FE + 1],
                             fl_s = Ac[FA_F * FE - BX], fl_n = Ac[FA_F * FE + BX];
                     const R f_m = Am[FA_F * FE], f_p = Ap[FA_F * FE];
@@ -428,8 +478,12 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
                 if (j == njm2) { su += an * hjp; sp -= an; an = R(0); }
                 if (i == 1) { su += aw * him; sp -= aw; aw = R(0); }
                 if (i == nim2) { su += ae * hip; sp -= ae; ae = R(0); }
-                R ap = an + as_ + ae + aw + at + ab + apnot - sp;
-                const R urfh = (R)p.urfh;
+                R ap;
+                if constexpr (kF32)  // fused in both forms of a cell, so that they give the same bits
+                    ap = fused(densbydt, vol, an + as_ + ae + aw + at + ab) - sp;
+                else
+                    ap = an + as_ + ae + aw + at + ab + apnot - sp;
+                const R urfh = cst.urfh;
                 ap = FAST ? ap * inv_urfh : bdiv(ap, urfh);
                 su += (R(1) - urfh) * ap * hc;
                 if constexpr (DC) {
@@ -459,6 +513,12 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
                 bl += (double)(ap - an - as_ - at - ab);
                 blp += (double)ae;
                 blm += (double)aw;
+            };
+            if (cell) {
+                if (CALM && still)
+                    interior(std::bool_constant<CALM>{});
+                else
+                    interior(std::false_type{});
             }
         }
         // this warp is done with planes k-1 (ring A) and k (ring B); the last warp
@@ -524,6 +584,23 @@ dim3 energy_assemble_grid(const Params &p, int kseg)
     return dim3((p.ni + kTX - 1) / kTX, (p.nj + kTY - 1) / kTY, (p.nk + seg - 1) / seg);
 }
 
+// The instantiations of a scheme, and the one for a grid of `ctas` CTAs (see the
+// kernel): 0 without the short form, 1 with it, 2 with it and four CTAs a SM (FP32).
+template <typename T, int SCH, bool DC> static auto assemble_variant(int v)
+{
+    constexpr int OCC = sizeof(T) == 4 ? 3 : 2, MORE = sizeof(T) == 4 ? 4 : 2;
+    return v == 0 ? energy_assemble_kernel<T, SCH, DC, false, OCC>
+         : v == 1 ? energy_assemble_kernel<T, SCH, DC, true, OCC> : energy_assemble_kernel<T, SCH, DC, true, MORE>;
+}
+template <typename T, int SCH> static void assemble_smem(int sm)
+{
+    for (int v = 0; v < 3; ++v) {
+        cudaFuncSetAttribute(assemble_variant<T, SCH, false>(v), cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+        if constexpr (sizeof(T) == sizeof(double))
+            cudaFuncSetAttribute(assemble_variant<T, SCH, true>(v), cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    }
+}
+
 // Tensor maps of the ten staged fields; set [q] reads diff/rho from the
 // buffers that are current at property parity q (parity 0: diff_a, rho_a).
 template <typename T> int make_assemble_maps(Inst<T> &I, T *diff_a, T *diff_b, T *rho_a, T *rho_b)
@@ -551,14 +628,9 @@ template <typename T> int make_assemble_maps(Inst<T> &I, T *diff_a, T *diff_b, T
     }
     I.asm_diff_a = diff_a;
     const int sm = (int)B::SMEM;
-    cudaFuncSetAttribute(energy_assemble_kernel<T, 0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    cudaFuncSetAttribute(energy_assemble_kernel<T, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    cudaFuncSetAttribute(energy_assemble_kernel<T, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    if constexpr (sizeof(T) == sizeof(double)) {
-        cudaFuncSetAttribute(energy_assemble_kernel<T, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-        cudaFuncSetAttribute(energy_assemble_kernel<T, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-        cudaFuncSetAttribute(energy_assemble_kernel<T, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    }
+    assemble_smem<T, 0>(sm);
+    assemble_smem<T, 1>(sm);
+    assemble_smem<T, 2>(sm);
     return 0;
 }
 
@@ -566,17 +638,16 @@ template <typename T, bool DC> static void assemble_scheme(Inst<T> &I, const Asm
 {
     const dim3 blk(kTX, kTY);
     const size_t sm = AsmBox<T>::SMEM;
-    switch (I.p.scheme) {
-    case AMCFD_SCHEME_UPWIND:
-        launch_k(I.pdl, energy_assemble_kernel<T, 0, DC>, I.asm_grid, blk, sm, I.stream, I.p, I.g, I.red_asm, m, I.dc);
-        break;
-    case AMCFD_SCHEME_POWER_LAW:
-        launch_k(I.pdl, energy_assemble_kernel<T, 1, DC>, I.asm_grid, blk, sm, I.stream, I.p, I.g, I.red_asm, m, I.dc);
-        break;
-    default:
-        launch_k(I.pdl, energy_assemble_kernel<T, 2, DC>, I.asm_grid, blk, sm, I.stream, I.p, I.g, I.red_asm, m, I.dc);
-        break;
-    }
+    const Params &p = I.p;
+    const AsmConst<T> cst = {(T)p.thconla, (T)p.thconlb, (T)p.acpl, (T)p.thconsa, (T)p.thconsb, (T)p.thconsc,
+                             (T)p.acpa, (T)p.acpb, (T)p.tliquid, (T)p.tsolid, (T)p.denl, (T)p.dens, (T)p.viscos,
+                             (T)p.urfh, (T)p.hlatnt, (T)(1.0 / p.acpl), (T)(1.0 / p.urfh)};
+    const long long ctas = (long long)I.asm_grid.x * I.asm_grid.y * I.asm_grid.z;
+    const int v = ctas <= I.sm_count ? 0 : ctas <= 3ll * I.sm_count ? 1 : 2;
+    const auto kern = p.scheme == AMCFD_SCHEME_UPWIND      ? assemble_variant<T, 0, DC>(v)
+                    : p.scheme == AMCFD_SCHEME_POWER_LAW ? assemble_variant<T, 1, DC>(v)
+                                                         : assemble_variant<T, 2, DC>(v);
+    launch_k(I.pdl, kern, I.asm_grid, blk, sm, I.stream, I.p, I.g, I.red_asm, m, I.dc, cst);
 }
 
 template <typename T> void launch_energy_assemble(Inst<T> &I)
