@@ -27,6 +27,7 @@ template <typename T> void set_sweep_smem_limit(size_t smem);
 template <typename T> int set_rounds_smem_limit(const Params &p);
 template <typename T> int setup_pipe_sweep(const Params &p, int warps, int sm_count, size_t &smem);
 template <typename T> bool setup_resident(const Params &p);
+template <typename T> size_t setup_rows(const Params &p, int sm_count, int &grid);
 dim3 energy_assemble_grid(const Params &p, int kseg);
 template <typename T> int h2t_blocks_per_sm();
 template <typename T> void launch_pack_field(const T *src, double *dst, int ni, int nip,
@@ -554,6 +555,10 @@ static int setup_instance(amcfd_ctx *ctx, Inst<T> &I)
         // or, on a domain small enough, with every line kept by a warp
         I.resident = (I.dc_on && !p.species) || setup_resident<T>(p);
         if (I.dc_on) I.resident = I.resident && setup_resident<float>(p);
+    }
+    if (I.order == AMCFD_ORDER_EXACT && !ctx->serial_launch) {
+        const size_t words = setup_rows<T>(p, I.sm_count, I.row_grid);
+        if (words > 0 && (rc = alloc3<unsigned long long>(ctx, &I.xrow, words))) return rc;
     }
     int bps = exact_sweep_blocks_per_sm<T>(I.exact_warps, I.line_smem);
     // A wave of the exact-order sweep holds about 2(nj-2)/3 lines; about three

@@ -20,6 +20,8 @@
 // mode runs visits in (t, m, s) order with per-line counters, reproducing the
 // reference iterates; the red-black mode updates all lines of one (j+k)
 // colour at once.
+#include <algorithm>
+
 #include "kernels.cuh"
 #include "amcfd.h"
 #include "async.cuh"
@@ -197,6 +199,298 @@ __global__ void sweep_exact_kernel(Params p, Fields<T> g, T *phi, int *flags, co
             atomicAdd(seqp, 1ull);
         }
     }
+}
+
+// ---------------------------------------------------------------------------
+// Exact-order sweep of the whole domain, a warp a row of visits.
+//
+// The reference's order is a wavefront (see the head of this file) whose depth,
+// 6M + J waves, times the latency of one visit is the solve's time: bytes and
+// arithmetic are a few per cent of it.  Handing out single visits cost 4.2 us a wave:
+// ticket, staging, four polls, the neighbour rows, and a fence before the line's
+// counter.  Here a warp takes a row, the visits (ks, k, s, j0..j1) of one plane and
+// j-sweep, and walks along j:
+//   * line j - 1 of the same sweep is its own last result, in registers;
+//   * the other neighbours' values carry their version: each cell has one 8-byte
+//     exchange word (FP32: value low, version high) or two (FP64: the value's halves,
+//     each under the version), so a reader that sees the version it wants in every
+//     word has the value: no fence and no counter.  Version v + 1 is what visit
+//     v = 2 ks + s leaves.  Visit v reads version v of line j + 1, version 2 ks + 2 of
+//     plane k + 1 and 2 ks of plane k - 1; version 0 is the unknown before the solve,
+//     which its line keeps in phi until its last visit.  A line goes on to its next
+//     visit only after these readers' own visits, so no version passes unseen.  The
+//     words of line j + 1 are loaded while line j is solved, and again if too early;
+//   * a second warp brings the coefficient rows of the next lines by bulk copies.
+// Rows are handed out by an atomic ticket in the order (ks, k, s), which every
+// dependency precedes: the smallest outstanding row is always runnable, so no
+// co-residency is assumed.  Waits are bounded (wait_polls).
+// The line arithmetic is solve_staged's and scan_line's: the same bits.
+// Measured (us a solve, FP64): 61x31x21 cells 635 -> 282, 120x60x40 1352 -> 879, 40x200x30
+// 1554 -> 577; FP32 100x48x30 957 -> 414.  A row lags the one before by one to two visits of
+// 1.3 us (scans 0.5, a word's way between SMs 0.3-0.5, the rest loads and stores).
+// ---------------------------------------------------------------------------
+template <typename T> constexpr int kRowW = (int)sizeof(T) / 4;  // exchange words a cell
+__device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long *p)
+{
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+// A cell's exchange words as loaded; their value if they hold version `tag`.
+template <typename T> struct RowWord;
+template <> struct RowWord<float> {
+    unsigned long long a;
+    __device__ __forceinline__ void load(const unsigned long long *xc, size_t c) { a = ld_relaxed_u64(xc + c); }
+    __device__ __forceinline__ bool holds(unsigned tag) const { return (unsigned)(a >> 32) == tag; }
+    __device__ __forceinline__ float value() const { return __uint_as_float((unsigned)a); }
+};
+template <> struct RowWord<double> {
+    unsigned long long a, b;
+    __device__ __forceinline__ void load(const unsigned long long *xc, size_t c)
+    {
+        asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(xc + 2 * c) : "memory");
+    }
+    __device__ __forceinline__ bool holds(unsigned tag) const
+    {
+        return (unsigned)(a >> 32) == tag && (unsigned)(b >> 32) == tag;
+    }
+    __device__ __forceinline__ double value() const { return __hiloint2double((int)(unsigned)b, (int)(unsigned)a); }
+};
+template <typename T>
+__device__ __forceinline__ bool row_load(const unsigned long long *xc, size_t c, unsigned tag, T &v)
+{
+    RowWord<T> w;
+    w.load(xc, c);
+    v = w.value();
+    return w.holds(tag);
+}
+__device__ __forceinline__ void row_store(unsigned long long *xc, size_t c, unsigned tag, float v)
+{
+    const unsigned long long w = ((unsigned long long)tag << 32) | __float_as_uint(v);
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(xc + c), "l"(w) : "memory");
+}
+__device__ __forceinline__ void row_store(unsigned long long *xc, size_t c, unsigned tag, double v)
+{
+    const unsigned long long t = (unsigned long long)tag << 32;
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(xc + 2 * c),
+                 "l"(t | (unsigned)__double2loint(v)), "l"(t | (unsigned)__double2hiint(v)) : "memory");
+}
+
+constexpr int kRowSlots = 4;  // lines whose coefficient rows a CTA holds
+// Dynamic shared memory of a CTA: the slots' rows, two mbarriers a slot.
+template <typename T> size_t rows_smem(const Params &p)
+{
+    return (size_t)kRowSlots * S_N * p.nip * sizeof(T) + 2 * kRowSlots * 8;
+}
+
+// L: cells a lane, (cells of a line + 31) / 32, kept in registers (two lines' neighbours at
+// a time, so at most four).
+template <typename T, int L>
+__global__ void __launch_bounds__(64) sweep_rows_kernel(Params p, Fields<T> g, T *phi, unsigned long long *xc)
+{
+    pdl_wait();
+    extern __shared__ __align__(128) unsigned char smraw[];
+    Status *st = g.st;
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int nmax = p.nip, nj = p.nj, nip = p.nip;
+    T *sl0 = reinterpret_cast<T *>(smraw);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(sl0 + (size_t)kRowSlots * S_N * nmax), *empty = bar + kRowSlots;
+    __shared__ unsigned long long row_of[8];  // the rows handed to the solving warp, in turn (at most kRowSlots + 1 ahead)
+    __shared__ uint32_t staged, solved;
+    __shared__ volatile int stop;
+    if (threadIdx.x < 2 * kRowSlots) mbar_init(bar + threadIdx.x);
+    if (threadIdx.x == 0) stop = 0;
+    __syncthreads();
+    const int i0 = 1, i1 = p.nim2, j0 = 1, j1 = p.njm2, k1 = p.nkm2, M = p.nkm2, n = i1;
+    const size_t sj = nip, sk = (size_t)nj * nip;
+    const unsigned tag0 = ((unsigned)*(volatile unsigned long long *)&st->seq_energy + 1u) * 8u;
+    int ib, ie;
+    stage_window<T>(i0, i1, ib, ie);
+    const int o = i0 - ib;
+    bool ok = !*(volatile int *)&st->error;
+    if (threadIdx.x >= 32) {
+        // ---- the other warp, one thread: rows' tickets, and their lines' coefficient rows
+        // kRowSlots lines ahead of the solving warp (issuing eight copies took a third
+        // of a visit there) ----
+        if (lane == 0) {
+            uint32_t f = 0;
+            auto slot_free = [&] {  // bounded by the solving warp's own waits
+                while (f >= kRowSlots && !mbar_try(empty + f % kRowSlots, (f / kRowSlots - 1) & 1u, 64))
+                    if (stop) return false;
+                return !stop;
+            };
+            for (uint32_t r = 0; slot_free(); ++r) {
+                const unsigned long long rk = ok ? atomicAdd(&st->ticket_energy, 1ull) : ~0ull;
+                row_of[r & 7] = rk;
+                if (rk >= 4ull * (unsigned)M) {
+                    mbar_arrive(bar + f % kRowSlots);
+                    ++f;
+                    break;
+                }
+                const int m = (int)(rk >> 1), k = k1 - (m >= M ? m - M : m);
+                int j = j0;
+                for (; j <= j1 && slot_free(); ++j, ++f)
+                    stage_line<T>(g, cidx(0, j, k, nj, nip), ib, ie, sl0 + (size_t)(f % kRowSlots) * S_N * nmax, nmax,
+                                  bar + f % kRowSlots);
+                if (j <= j1) break;
+            }
+            staged = f;
+        }
+        __syncwarp();
+    } else {
+        // ---- the solving warp ----
+        uint32_t used = 0;  // lines solved so far: line f is in slot f % kRowSlots
+        auto line_ready = [&]() { return __all_sync(full, mbar_wait(bar + used % kRowSlots, (used / kRowSlots) & 1u, st, -8)) != 0; };
+        auto line_done = [&]() {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(empty + used % kRowSlots);
+            ++used;
+        };
+        long long it = 0;  // polls of the current wait
+        // one poll of the warp has run without success: false when to give up
+        auto again = [&](int where) {
+            if ((it & 63) == 63 && __any_sync(full, *(volatile int *)&st->error != 0)) return false;
+            if (it++ > p.wait_polls) {
+                if (lane == 0 && atomicCAS(&st->error, 0, AMCFD_E_TIMEOUT) == 0) st->error_where = where;
+                return false;
+            }
+            return true;
+        };
+        for (uint32_t r = 0;; ++r) {
+            if (!line_ready()) { ok = false; break; }
+            const unsigned long long rk = row_of[r & 7];
+            if (rk >= 4ull * (unsigned)M) { ++used; break; }
+            const int m = (int)(rk >> 1), s = (int)(rk & 1), ks = m / M, k = k1 - (m - ks * M), v = 2 * ks + s;
+            const bool top = k < k1, bot = k > 1;
+            // versions of the neighbours above, below and north; 0: phi itself
+            const unsigned vt = top ? 2 * ks + 2 : 0, vb = bot ? 2 * ks : 0;
+            const int a = lane * L;
+            // line j's neighbours above, below and north: loads issued a line ahead, looked at
+            // when the line's turn comes (a version that was not there yet is loaded again)
+            struct Nb {
+                RowWord<T> w[3][L];
+                T val[3][L], lo, hi;
+            };
+            const long long off[3] = {(long long)sk, -(long long)sk, (long long)sj};
+            int at[L];  // this lane's cells in a row
+#pragma unroll
+            for (int c = 0; c < L; ++c) at[c] = a + c < n ? a + c : 0;
+            auto issue = [&](Nb &q, size_t row, bool north) {
+                const unsigned ver[3] = {vt, vb, north ? (unsigned)v : 0u};
+                q.lo = __ldcg(phi + row - 1);
+                q.hi = __ldcg(phi + row + n);
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+#pragma unroll
+                    for (int c = 0; c < L; ++c) {
+                        if (ver[d]) q.w[d][c].load(xc, row + at[c] + off[d]);
+                        else q.val[d][c] = __ldcg(phi + row + at[c] + off[d]);
+                    }
+            };
+            // what was not there yet, loaded again
+            auto reload = [&](Nb &q, size_t row, bool north) {
+                const unsigned ver[3] = {vt, vb, north ? (unsigned)v : 0u};
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+#pragma unroll
+                    for (int c = 0; c < L; ++c)
+                        if (ver[d] && !q.w[d][c].holds(tag0 + ver[d])) q.w[d][c].load(xc, row + at[c] + off[d]);
+            };
+            // true for the whole warp once every version is there
+            auto arrived = [&](const Nb &q, bool north) {
+                const unsigned ver[3] = {vt, vb, north ? (unsigned)v : 0u};
+                bool all = true;
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+#pragma unroll
+                    for (int c = 0; c < L; ++c)
+                        all = all && (!ver[d] || a + c >= n || q.w[d][c].holds(tag0 + ver[d]));
+                return __all_sync(full, all) != 0;
+            };
+            auto value = [&](const Nb &q, int d, int c, unsigned ver) { return ver ? q.w[d][c].value() : q.val[d][c]; };
+            T x[L];  // the line before
+            {
+                const size_t row = cidx(i0, j0 - 1, k, nj, nip);
+#pragma unroll
+                for (int c = 0; c < L; ++c) x[c] = __ldcg(phi + row + (a + c < n ? a + c : 0));
+            }
+            Nb cur, nxt;
+            size_t row = cidx(i0, j0, k, nj, nip);  // the line's first cell
+            issue(cur, row, j0 < j1);
+#pragma unroll 1
+            for (int j = j0; j <= j1; ++j, row += sj) {
+                it = 0;
+                // a plane of one line: its visits depend on nothing of one another, but their
+                // versions must land in turn
+                if (j0 == j1 && v > 0)
+                    for (;;) {
+                        bool turn = true;
+#pragma unroll
+                        for (int c = 0; c < L; ++c) {
+                            T y;
+                            turn = turn && (a + c >= n || row_load(xc, row + a + c, tag0 + (unsigned)v, y));
+                        }
+                        if (__all_sync(full, turn) || !(ok = again(k * nj + j))) break;
+                    }
+                while (ok && !arrived(cur, j < j1)) {
+                    reload(cur, row, j < j1);
+                    ok = again(k * nj + j);
+                }
+                if (!ok) break;
+                if (!(ok = line_ready())) break;
+                const T *sl = sl0 + (size_t)(used % kRowSlots) * S_N * nmax + o;
+                T e[L], cf[L], pr[L];
+#pragma unroll
+                for (int c = 0; c < L; ++c) {
+                    const int w = a + c < n ? a + c : 0;
+                    e[c] = line_rhs(sl[S_AT * nmax + w], value(cur, 0, c, vt), sl[S_AB * nmax + w],
+                                    value(cur, 1, c, vb), sl[S_AN * nmax + w], value(cur, 2, c, j < j1 ? v : 0),
+                                    sl[S_AS * nmax + w], x[c], sl[S_SU * nmax + w], sl[S_ID * nmax + w]);
+                    cf[c] = sl[S_CF * nmax + w];
+                    pr[c] = sl[S_PR * nmax + w];
+                }
+                // the next line's neighbours start while this line is solved
+                if (j < j1) issue(nxt, row + sj, j + 1 < j1);
+                scan_line_lanes<T, L>(n, e, cf, pr, cur.lo, cur.hi);
+                if (j < j1) reload(nxt, row + sj, j + 1 < j1);
+#pragma unroll
+                for (int c = 0; c < L; ++c) {
+                    x[c] = e[c];
+                    if (a + c < n) {
+                        if (v < 3 || bot) row_store(xc, row + a + c, tag0 + (unsigned)v + 1u, e[c]);
+                        if (v == 3) phi[row + a + c] = e[c];
+                    }
+                }
+                line_done();
+                cur = nxt;
+            }
+            if (!ok) break;
+        }
+        if (lane == 0) {
+            solved = used;
+            stop = 1;  // (a run that ends well has taken the last row already)
+        }
+    }
+    __syncthreads();
+    // after a failed wait: the copies still in flight land before the CTA's shared memory
+    // goes (bounded)
+    if (threadIdx.x == 0)
+        for (uint32_t f = solved; f < staged; ++f) mbar_try(bar + f % kRowSlots, (f / kRowSlots) & 1u, kSpinLimit);
+    pdl_release();
+    if (threadIdx.x == 0 && atomicAdd(&st->done_energy, 1ull) == (unsigned long long)gridDim.x - 1) {
+        // last CTA of this launch: reset the counters for the next one
+        atomicExch(&st->done_energy, 0ull);
+        atomicExch(&st->ticket_energy, 0ull);
+        __threadfence();
+        atomicAdd(&st->seq_energy, 1ull);
+    }
+}
+template <typename T> static auto rows_kernel(const Params &p)
+{
+    const int L = (p.nim2 + 31) / 32;
+    return L == 1 ? sweep_rows_kernel<T, 1> : L == 2 ? sweep_rows_kernel<T, 2> : L == 3 ? sweep_rows_kernel<T, 3>
+                                             : sweep_rows_kernel<T, 4>;
 }
 
 // ---------------------------------------------------------------------------
@@ -1265,6 +1559,8 @@ template <typename T> static void sweeps(Inst<T> &I, T *phi, bool box)
             sweep_exact_kernel<T, true><<<I.exact_grid, 32 * warps, smem, I.stream>>>(
                 I.p, I.g, phi, I.flags_mom, I.g.tickets_mom, 0, &st->seq_mom, &st->done_mom,
                 &st->ticket_mom);
+        else if (I.xrow)
+            launch_k(I.pdl, rows_kernel<T>(I.p), I.row_grid, 64, rows_smem<T>(I.p), I.stream, I.p, I.g, phi, I.xrow);
         else
             sweep_exact_kernel<T, false><<<I.exact_grid, 32 * warps, smem, I.stream>>>(
                 I.p, I.g, phi, I.g.flags, I.g.tickets_energy, I.g.ntickets_energy,
@@ -1410,6 +1706,25 @@ template <typename T> void set_sweep_smem_limit(size_t smem)
     raise_smem_limit((const void *)sweep_exact_kernel<T, true>, smem);
     raise_smem_limit((const void *)sweep_rb_kernel<T, true>, smem);
 }
+// Exact-order sweep by rows: the exchange words it needs (0 for lines past 128 cells, where
+// one warp a row fell behind the visits dealt out singly: 1960 against 1930 us a solve on
+// 160x80x50 cells, 4740 against 3460 on 300x150x60), with its shared-memory limit raised; `grid` receives its
+// (one-warp) CTAs: the rows a wave touches, 2 in 3 of a plane's lines, and a few that
+// wait, at most the rows there are and what is resident at once.
+template <typename T> size_t setup_rows(const Params &p, int sm_count, int &grid)
+{
+    const size_t need = rows_smem<T>(p);
+    int nb = 0;
+    if (p.nim2 > 128) return 0;
+    if (need > 200 * 1024 || raise_smem_limit((const void *)rows_kernel<T>(p), need) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rows_kernel<T>(p), 64, need) != cudaSuccess || nb < 1) {
+        cudaGetLastError();
+        return 0;
+    }
+    grid = std::max(1, std::min({4 * (p.nk_alloc - 2), 2 * (p.nj - 2) / 3 + 16, nb * sm_count}));
+    return (size_t)p.nk_alloc * p.nj * p.nip * kRowW<T>;
+}
+
 // The whole-domain red-black kernel's buffer (qr and pr of each warp's line): the
 // most warps per CTA (8, 4 or 2) whose buffers fit 200 KiB, with the limit raised
 // for them; 0 when not even 2 fit.
@@ -1441,6 +1756,7 @@ template <typename T> int setup_pipe_sweep(const Params &p, int warps, int sm_co
 
 #define AMCFD_INST(T)                                                     \
     template int setup_pipe_sweep<T>(const Params &, int, int, size_t &); \
+    template size_t setup_rows<T>(const Params &, int, int &);            \
     template bool setup_resident<T>(const Params &);                      \
     template void launch_energy_factor<T>(Inst<T> &);                    \
     template void launch_box_factor<T>(Inst<T> &);                       \

@@ -102,6 +102,10 @@ struct Inst {
     dim3 asm_grid;
     int grid_1d = 0;          // grid of the pointwise kernels
     int exact_grid = 0;       // CTAs of the persistent exact-order line sweep
+    // the exact-order sweep of the whole domain by rows: exchange words (null: by single
+    // visits) and CTAs of one warp
+    unsigned long long *xrow = nullptr;
+    int row_grid = 0;
     int exact_warps = 4;      // warps per CTA in the line sweeps
     size_t line_smem = 0;     // dynamic smem of a line-sweep CTA
     int *flags_mom = nullptr;

@@ -59,14 +59,12 @@ __device__ __forceinline__ void stage_line(const Fields<T> &g, size_t row, int i
 // by i - i0: e (right-hand side / den on entry, the solution on exit), cf and
 // pr.  Each lane owns a contiguous chunk; the chunks are chained by warp scans
 // of affine maps (x -> A x + B), forward for qr_i = cf_i qr_{i-1} + e_i and
-// backward for phi_i = pr_i phi_{i+1} + qr_i; then the line is stored.  lo and
+// backward for phi_i = pr_i phi_{i+1} + qr_i; the solution replaces e.  lo and
 // hi are the fixed end values phi_{i0-1} and phi_{i1+1}.
 template <typename T>
-__device__ __forceinline__ void scan_line(T *phi, size_t row, int i0, int i1, T *se, const T *sc,
-                                          const T *sp, T lo, T hi)
+__device__ __forceinline__ void scan_line_shared(int n, T *se, const T *sc, const T *sp, T lo, T hi)
 {
     const int lane = threadIdx.x & 31;
-    const int n = i1 - i0 + 1;
     const int L = (n + 31) >> 5;
     const int a = lane * L;
     const int b = min(a + L, n);
@@ -117,6 +115,15 @@ __device__ __forceinline__ void scan_line(T *phi, size_t row, int i0, int i1, T 
         x = fma_rn(sp[i], x, se[i]);
         se[i] = x;
     }
+}
+// The same, and the line stored.
+template <typename T>
+__device__ __forceinline__ void scan_line(T *phi, size_t row, int i0, int i1, T *se, const T *sc,
+                                          const T *sp, T lo, T hi)
+{
+    const int lane = threadIdx.x & 31;
+    const int n = i1 - i0 + 1;
+    scan_line_shared<T>(n, se, sc, sp, lo, hi);
     __syncwarp();
     for (int i = lane; i < n; i += 32) phi[row + i0 + i] = se[i];
 }
@@ -176,38 +183,20 @@ template <typename T, int L>
 struct LineRegs {
     T at[L], ab[L], an[L], as[L], su[L], cf[L], pr[L], id[L];
 };
-// One pass over a line of n <= 32 L cells from its registers: solve_staged and
-// scan_line with the same expressions on the same per-lane chunks (so the same
-// bits), the right-hand side and both recurrences in registers; only the four
-// neighbouring rows and the two fixed ends are read (through L2: other CTAs
-// write them), and the lane's cells are stored.
+// The recurrences of scan_line on a lane's cells in registers (cells lane L .. lane L + L - 1
+// of n <= 32 L; L = (n + 31) / 32 gives scan_line's chunks, so its bits): e is the
+// right-hand side on entry, the solution on exit.
 template <typename T, int L>
-__device__ __forceinline__ void solve_line_regs(T *phi, size_t row, int i0, int n, size_t sj, size_t sk,
-                                                const LineRegs<T, L> &r)
+__device__ __forceinline__ void scan_line_lanes(int n, T (&e)[L], const T (&cf)[L], const T (&pr)[L], T lo, T hi)
 {
     const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int a = lane * L;
-    const T lo = ld_shared_row<T>(phi + row + i0 - 1), hi = ld_shared_row<T>(phi + row + i0 + n);
-    T nt[L], nb[L], nn[L], ns[L], e[L];
-#pragma unroll
-    for (int v = 0; v < L; ++v) {
-        const bool ok = a + v < n;
-        const size_t c = row + i0 + (ok ? a + v : 0);
-        nt[v] = ok ? ld_shared_row<T>(phi + c + sk) : T(0);
-        nb[v] = ok ? ld_shared_row<T>(phi + c - sk) : T(0);
-        nn[v] = ok ? ld_shared_row<T>(phi + c + sj) : T(0);
-        ns[v] = ok ? ld_shared_row<T>(phi + c - sj) : T(0);
-    }
-#pragma unroll
-    for (int v = 0; v < L; ++v)
-        e[v] = line_rhs(r.at[v], nt[v], r.ab[v], nb[v], r.an[v], nn[v], r.as[v], ns[v], r.su[v], r.id[v]);
+    const int lane = threadIdx.x & 31, a = lane * L;
     T A = T(1), B = T(0);
 #pragma unroll
     for (int v = 0; v < L; ++v)
         if (a + v < n) {
-            B = fma_rn(r.cf[v], B, e[v]);
-            A = mul_rn(r.cf[v], A);
+            B = fma_rn(cf[v], B, e[v]);
+            A = mul_rn(cf[v], A);
         }
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -225,7 +214,7 @@ __device__ __forceinline__ void solve_line_regs(T *phi, size_t row, int i0, int 
 #pragma unroll
     for (int v = 0; v < L; ++v)
         if (a + v < n) {
-            q = fma_rn(r.cf[v], q, e[v]);
+            q = fma_rn(cf[v], q, e[v]);
             e[v] = q;
         }
     A = T(1);
@@ -233,8 +222,8 @@ __device__ __forceinline__ void solve_line_regs(T *phi, size_t row, int i0, int 
 #pragma unroll
     for (int v = L - 1; v >= 0; --v)
         if (a + v < n) {
-            B = fma_rn(r.pr[v], B, e[v]);
-            A = mul_rn(r.pr[v], A);
+            B = fma_rn(pr[v], B, e[v]);
+            A = mul_rn(pr[v], A);
         }
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -252,9 +241,39 @@ __device__ __forceinline__ void solve_line_regs(T *phi, size_t row, int i0, int 
 #pragma unroll
     for (int v = L - 1; v >= 0; --v)
         if (a + v < n) {
-            x = fma_rn(r.pr[v], x, e[v]);
-            phi[row + i0 + a + v] = x;
+            x = fma_rn(pr[v], x, e[v]);
+            e[v] = x;
         }
+}
+// One pass over a line of n <= 32 L cells from its registers: solve_staged and
+// scan_line with the same expressions on the same per-lane chunks (so the same
+// bits), the right-hand side and both recurrences in registers; only the four
+// neighbouring rows and the two fixed ends are read (through L2: other CTAs
+// write them), and the lane's cells are stored.
+template <typename T, int L>
+__device__ __forceinline__ void solve_line_regs(T *phi, size_t row, int i0, int n, size_t sj, size_t sk,
+                                                const LineRegs<T, L> &r)
+{
+    const int lane = threadIdx.x & 31;
+    const int a = lane * L;
+    const T lo = ld_shared_row<T>(phi + row + i0 - 1), hi = ld_shared_row<T>(phi + row + i0 + n);
+    T nt[L], nb[L], nn[L], ns[L], e[L];
+#pragma unroll
+    for (int v = 0; v < L; ++v) {
+        const bool ok = a + v < n;
+        const size_t c = row + i0 + (ok ? a + v : 0);
+        nt[v] = ok ? ld_shared_row<T>(phi + c + sk) : T(0);
+        nb[v] = ok ? ld_shared_row<T>(phi + c - sk) : T(0);
+        nn[v] = ok ? ld_shared_row<T>(phi + c + sj) : T(0);
+        ns[v] = ok ? ld_shared_row<T>(phi + c - sj) : T(0);
+    }
+#pragma unroll
+    for (int v = 0; v < L; ++v)
+        e[v] = line_rhs(r.at[v], nt[v], r.ab[v], nb[v], r.an[v], nn[v], r.as[v], ns[v], r.su[v], r.id[v]);
+    scan_line_lanes<T, L>(n, e, r.cf, r.pr, lo, hi);
+#pragma unroll
+    for (int v = 0; v < L; ++v)
+        if (a + v < n) phi[row + i0 + a + v] = e[v];
 }
 
 // ---------------------------------------------------------------------------
