@@ -160,190 +160,216 @@ template <typename T> struct CellEq {
     T an, as, ae, aw, at, ab, ap, su, d, pt, pb, pn, ps;
 };
 
-// One cell of the u/v/w equation (ivar 1..3) of the momentum box: coefficients,
-// source, under-relaxation, the solid freeze and d = A/ap; returns |residual| of
-// the cell (calculateResiduals(1..3)).
-template <typename T, class LD>
-__device__ __forceinline__ double mom_cell_eq(const Params &p, const Fields<T> &g, const Status *st, int ivar, int i,
-                                              int j, int k, CellEq<T> &q)
+// What a cell's u/v/w equation needs besides the flow: face conductances and
+// viscosities (n, s, e, w, t, b), face areas, volume, the transient coefficient, the Darcy
+// and buoyancy terms.  It depends on the iteration's properties and temperatures only,
+// so a launch that has threads to spare can form it before the flow is known.
+template <typename T> struct CellPre {
+    T dn, ds, de, dw, dt, db, vn, vs, ve, vw, vt, vb;
+    T a1, a2, a3, vol, rc, apnot;  // areas: faces in j, in i, in k
+    T term, bv, dtw;               // Darcy coefficient; buoyancy: coefficient x volume, T - T_solidus
+    T flags;                       // 1: some liquid, + 2: frozen
+};
+
+template <typename T>
+__device__ __forceinline__ void mom_cell_pre(const Params &p, const Fields<T> &g, const Status *st, int ivar, int i,
+                                             int j, int k, CellPre<T> &q)
 {
     using R = T;
     const int nj = p.nj, nip = p.nip, nkm2 = p.nkm2, njm2 = p.njm2, nim2 = p.nim2;
     const size_t sj = nip, sk = (size_t)nj * nip;
-    const int sch = p.scheme;
     const R delt = (R)st->delt;
-    const LD u{g.uvel}, v{g.vvel}, w{g.wvel};
     const R *rho = g.rho_nxt, *vis = g.vis_nxt;
     const double *fx = g.fracx, *fy = g.fracy, *fz = g.fracz, *xu = g.xu, *yv = g.yv, *zw = g.zw;
     const size_t c = cidx(i, j, k, nj, nip);
-    R an, as_, ae, aw, at, ab, apnot, su, sp, tmp, areaD, vol;
     const R rc = rho[c];
-    LD phi;
     size_t cn;  // upstream scalar node of the staggered cell
-    R urf, flv;
+    R flv;
+    q.bv = q.dtw = R(0);
     if (ivar == 1) {
         const R fxm = (R)fx[i - 1];
-        R vn = v[c + sj] * (R(1) - fxm) + v[c + sj - 1] * fxm;
-        R vs = v[c] * (R(1) - fxm) + v[c - 1] * fxm;
-        R ue = (u[c + 1] + u[c]) * R(0.5);
-        R uw = (u[c - 1] + u[c]) * R(0.5);
-        R wt = w[c + sk] * (R(1) - fxm) + w[c + sk - 1] * fxm;
-        R wb = w[c] * (R(1) - fxm) + w[c - 1] * fxm;
         const R auik = (R)area_uik(g, i, k), ajk = (R)area_jk(p, g, j, k), auij = (R)area_uij(g, i, j);
-        R fn = vn * rc * auik, fs = vs * rc * auik, fe = ue * rc * ajk, fw = uw * rc * ajk;
-        R ft = wt * rc * auij, fb = wb * rc * auij;
         R visu = vis[c] * vis[c - 1] / (fxm * vis[c - 1] + (R(1) - fxm) * vis[c]);
         R visun = vis[c + sj] * vis[c + sj - 1] / (fxm * vis[c + sj - 1] + (R(1) - fxm) * vis[c + sj]);
         R visus = vis[c - sj] * vis[c - sj - 1] / (fxm * vis[c - sj - 1] + (R(1) - fxm) * vis[c - sj]);
-        R visn = (j == njm2) ? visu : visu * visun / ((R(1) - (R)fy[j]) * visun + (R)fy[j] * visu);
-        R viss = (j == 1) ? visu : visu * visus / ((R)fy[j - 1] * visus + (R(1) - (R)fy[j - 1]) * visu);
-        R vise = vis[c], visw = vis[c - 1];
+        q.vn = (j == njm2) ? visu : visu * visun / ((R(1) - (R)fy[j]) * visun + (R)fy[j] * visu);
+        q.vs = (j == 1) ? visu : visu * visus / ((R)fy[j - 1] * visus + (R(1) - (R)fy[j - 1]) * visu);
+        q.ve = vis[c];
+        q.vw = vis[c - 1];
         R visut = vis[c + sk] * vis[c + sk - 1] / (fxm * vis[c + sk - 1] + (R(1) - fxm) * vis[c + sk]);
         R visub = vis[c - sk] * vis[c - sk - 1] / (fxm * vis[c - sk - 1] + (R(1) - fxm) * vis[c - sk]);
-        R vist = (k == nkm2) ? visu : visut * visu / ((R)fz[k] * visu + (R(1) - (R)fz[k]) * visut);
-        R visb = (k == 1) ? visu : visub * visu / ((R(1) - (R)fz[k - 1]) * visu + (R)fz[k - 1] * visub);
-        R dn = visn * auik * (R)g.dypsinv[j + 1], ds = viss * auik * (R)g.dypsinv[j];
-        R de = vise * ajk / (R)(xu[i + 1] - xu[i]), dw = visw * ajk / (R)(xu[i] - xu[i - 1]);
-        R dt = vist * auij * (R)g.dzpbinv[k + 1], db = visb * auij * (R)g.dzpbinv[k];
-        face_coef<R>(sch, dn, fn, an, tmp);
-        face_coef<R>(sch, ds, fs, tmp, as_);
-        face_coef<R>(sch, de, fe, ae, tmp);
-        face_coef<R>(sch, dw, fw, tmp, aw);
-        face_coef<R>(sch, dt, ft, at, tmp);
-        face_coef<R>(sch, db, fb, tmp, ab);
-        vol = (R)volume_u(g, i, j, k);
-        apnot = rc * vol / delt;
-        R delf = fn - fs + fe - fw + ft - fb;
-        R cp0 = maxd(R(0), delf), cp1 = mind(R(0), delf);
-        su = -cp1 * u[c];
-        su += ajk * (g.pressure[c - 1] - g.pressure[c]);
-        sp = -cp0;
-        su += apnot * g.unot[c];
-        R dudxp = (u[c + 1] - u[c]) / (R)(xu[i + 1] - xu[i]);
-        R dudxm = (u[c] - u[c - 1]) / (R)(xu[i] - xu[i - 1]);
-        su += (vise * dudxp - visw * dudxm) * ajk;
-        R dvdxp = (v[c + sj] - v[c + sj - 1]) * (R)g.dxpwinv[i];
-        R dvdxm = (v[c] - v[c - 1]) * (R)g.dxpwinv[i];
-        su += (visn * dvdxp - viss * dvdxm) * auik;
-        R dwdxp = (w[c + sk] - w[c + sk - 1]) * (R)g.dxpwinv[i];
-        R dwdxm = (w[c] - w[c - 1]) * (R)g.dxpwinv[i];
-        su += (vist * dwdxp - visb * dwdxm) * auij;
-        phi = u; cn = c - 1; urf = (R)p.urfu; areaD = ajk;
+        q.vt = (k == nkm2) ? visu : visut * visu / ((R)fz[k] * visu + (R(1) - (R)fz[k]) * visut);
+        q.vb = (k == 1) ? visu : visub * visu / ((R(1) - (R)fz[k - 1]) * visu + (R)fz[k - 1] * visub);
+        q.dn = q.vn * auik * (R)g.dypsinv[j + 1];
+        q.ds = q.vs * auik * (R)g.dypsinv[j];
+        q.de = q.ve * ajk / (R)(xu[i + 1] - xu[i]);
+        q.dw = q.vw * ajk / (R)(xu[i] - xu[i - 1]);
+        q.dt = q.vt * auij * (R)g.dzpbinv[k + 1];
+        q.db = q.vb * auij * (R)g.dzpbinv[k];
+        q.a1 = auik; q.a2 = ajk; q.a3 = auij;
+        q.vol = (R)volume_u(g, i, j, k);
+        cn = c - 1;
         flv = g.fracl[c] * (R(1) - fxm) + g.fracl[c - 1] * fxm;
     } else if (ivar == 2) {
         const R fym = (R)fy[j - 1];
-        R vn = (v[c] + v[c + sj]) * R(0.5);
-        R vs = (v[c] + v[c - sj]) * R(0.5);
-        R ue = u[c + 1] * (R(1) - fym) + u[c + 1 - sj] * fym;
-        R uw = u[c] * (R(1) - fym) + u[c - sj] * fym;
-        R wt = w[c + sk] * (R(1) - fym) + w[c + sk - sj] * fym;
-        R wb = w[c] * (R(1) - fym) + w[c - sj] * fym;
         const R aik = (R)area_ik(p, g, i, k), avjk = (R)area_vjk(g, j, k), avij = (R)area_vij(g, i, j);
-        R fn = vn * rc * aik, fs = vs * rc * aik, fe = ue * rc * avjk, fw = uw * rc * avjk;
-        R ft = wt * rc * avij, fb = wb * rc * avij;
-        R visn = vis[c], viss = vis[c - sj];
+        q.vn = vis[c];
+        q.vs = vis[c - sj];
         R visv = vis[c] * vis[c - sj] / (fym * vis[c - sj] + (R(1) - fym) * vis[c]);
         R visve = vis[c + 1] * vis[c + 1 - sj] / (fym * vis[c + 1 - sj] + (R(1) - fym) * vis[c + 1]);
         R visvw = vis[c - 1] * vis[c - 1 - sj] / (fym * vis[c - 1 - sj] + (R(1) - fym) * vis[c - 1]);
-        R vise = (i == nim2) ? visv : visv * visve / ((R(1) - (R)fx[i]) * visve + (R)fx[i] * visv);
-        R visw = (i == 1) ? visv : visv * visvw / ((R)fx[i - 1] * visvw + (R(1) - (R)fx[i - 1]) * visv);
+        q.ve = (i == nim2) ? visv : visv * visve / ((R(1) - (R)fx[i]) * visve + (R)fx[i] * visv);
+        q.vw = (i == 1) ? visv : visv * visvw / ((R)fx[i - 1] * visvw + (R(1) - (R)fx[i - 1]) * visv);
         R visvt = vis[c + sk] * vis[c + sk - sj] / (fym * vis[c + sk - sj] + (R(1) - fym) * vis[c + sk]);
         R visvb = vis[c - sk] * vis[c - sk - sj] / (fym * vis[c - sk - sj] + (R(1) - fym) * vis[c - sk]);
-        R vist = (k == nkm2) ? visv : visv * visvt / ((R(1) - (R)fz[k]) * visvt + (R)fz[k] * visv);
-        R visb = (k == 1) ? visv : visv * visvb / ((R)fz[k - 1] * visvb + (R(1) - (R)fz[k - 1]) * visv);
-        R dn = visn * aik / (R)(yv[j + 1] - yv[j]), ds = viss * aik / (R)(yv[j] - yv[j - 1]);
-        R de = vise * avjk * (R)g.dxpwinv[i + 1], dw = visw * avjk * (R)g.dxpwinv[i];
-        R dt = vist * avij * (R)g.dzpbinv[k + 1], db = visb * avij * (R)g.dzpbinv[k];
-        face_coef<R>(sch, dn, fn, an, tmp);
-        face_coef<R>(sch, ds, fs, tmp, as_);
-        face_coef<R>(sch, de, fe, ae, tmp);
-        face_coef<R>(sch, dw, fw, tmp, aw);
-        face_coef<R>(sch, dt, ft, at, tmp);
-        face_coef<R>(sch, db, fb, tmp, ab);
-        vol = (R)volume_v(g, i, j, k);
-        apnot = rc * vol / delt;
-        R delf = fn - fs + fe - fw + ft - fb;
-        R cp0 = maxd(R(0), delf), cp1 = mind(R(0), delf);
-        su = -cp1 * v[c];
-        su += aik * (g.pressure[c - sj] - g.pressure[c]);
-        sp = -cp0;
-        su += apnot * g.vnot[c];
-        R dudyp = (u[c + 1] - u[c + 1 - sj]) * (R)g.dypsinv[j];
-        R dudym = (u[c] - u[c - sj]) * (R)g.dypsinv[j];
-        su += (vise * dudyp - visw * dudym) * avjk;
-        R dvdyp = (v[c + sj] - v[c]) / (R)(yv[j + 1] - yv[j]);
-        R dvdym = (v[c] - v[c - sj]) / (R)(yv[j] - yv[j - 1]);
-        su += (visn * dvdyp - viss * dvdym) * aik;
-        R dwdyp = (w[c + sk] - w[c + sk - sj]) * (R)g.dypsinv[j];
-        R dwdym = (w[c] - w[c - sj]) * (R)g.dypsinv[j];
-        su += (vist * dwdyp - visb * dwdym) * avij;
-        phi = v; cn = c - sj; urf = (R)p.urfv; areaD = aik;
+        q.vt = (k == nkm2) ? visv : visv * visvt / ((R(1) - (R)fz[k]) * visvt + (R)fz[k] * visv);
+        q.vb = (k == 1) ? visv : visv * visvb / ((R)fz[k - 1] * visvb + (R(1) - (R)fz[k - 1]) * visv);
+        q.dn = q.vn * aik / (R)(yv[j + 1] - yv[j]);
+        q.ds = q.vs * aik / (R)(yv[j] - yv[j - 1]);
+        q.de = q.ve * avjk * (R)g.dxpwinv[i + 1];
+        q.dw = q.vw * avjk * (R)g.dxpwinv[i];
+        q.dt = q.vt * avij * (R)g.dzpbinv[k + 1];
+        q.db = q.vb * avij * (R)g.dzpbinv[k];
+        q.a1 = aik; q.a2 = avjk; q.a3 = avij;
+        q.vol = (R)volume_v(g, i, j, k);
+        cn = c - sj;
         flv = g.fracl[c] * (R(1) - fym) + g.fracl[c - sj] * fym;
     } else {
         const R fzm = (R)fz[k - 1];
-        R vn = v[c + sj] * (R(1) - fzm) + v[c + sj - sk] * fzm;
-        R vs = v[c] * (R(1) - fzm) + v[c - sk] * fzm;
-        R ue = u[c + 1] * (R(1) - fzm) + u[c + 1 - sk] * fzm;
-        R uw = u[c] * (R(1) - fzm) + u[c - sk] * fzm;
-        R wt = (w[c] + w[c + sk]) * R(0.5);
-        R wb = (w[c] + w[c - sk]) * R(0.5);
         const R awik = (R)area_wik(g, i, k), awjk = (R)area_wjk(g, j, k), aij = (R)area_ij(p, g, i, j);
-        R fn = vn * rc * awik, fs = vs * rc * awik, fe = ue * rc * awjk, fw = uw * rc * awjk;
-        R ft = wt * rc * aij, fb = wb * rc * aij;
         R vis_w = vis[c] * vis[c - sk] / (fzm * vis[c - sk] + (R(1) - fzm) * vis[c]);
         R viswn = vis[c + sj] * vis[c + sj - sk] / (fzm * vis[c + sj - sk] + (R(1) - fzm) * vis[c + sj]);
         R visws = vis[c - sj] * vis[c - sj - sk] / (fzm * vis[c - sj - sk] + (R(1) - fzm) * vis[c - sj]);
-        R visn = (j == njm2) ? vis_w : vis_w * viswn / ((R(1) - (R)fy[j]) * viswn + (R)fy[j] * vis_w);
-        R viss = (j == 1) ? vis_w : vis_w * visws / ((R)fy[j - 1] * visws + (R(1) - (R)fy[j - 1]) * vis_w);
+        q.vn = (j == njm2) ? vis_w : vis_w * viswn / ((R(1) - (R)fy[j]) * viswn + (R)fy[j] * vis_w);
+        q.vs = (j == 1) ? vis_w : vis_w * visws / ((R)fy[j - 1] * visws + (R(1) - (R)fy[j - 1]) * vis_w);
         R viswe = vis[c + 1] * vis[c + 1 - sk] / (fzm * vis[c + 1 - sk] + (R(1) - fzm) * vis[c + 1]);
         R visww = vis[c - 1] * vis[c - 1 - sk] / (fzm * vis[c - 1 - sk] + (R(1) - fzm) * vis[c - 1]);
-        R vise = (i == nim2) ? vis_w : vis_w * viswe / ((R(1) - (R)fx[i]) * viswe + (R)fx[i] * vis_w);
-        R visw = (i == 1) ? vis_w : vis_w * visww / ((R)fx[i - 1] * visww + (R(1) - (R)fx[i - 1]) * vis_w);
-        R vist = vis[c], visb = vis[c - sk];
-        R dn = visn * awik * (R)g.dypsinv[j + 1], ds = viss * awik * (R)g.dypsinv[j];
-        R de = vise * awjk * (R)g.dxpwinv[i + 1], dw = visw * awjk * (R)g.dxpwinv[i];
-        R dt = vist * aij / (R)(zw[k + 1] - zw[k]), db = visb * aij / (R)(zw[k] - zw[k - 1]);
-        face_coef<R>(sch, dn, fn, an, tmp);
-        face_coef<R>(sch, ds, fs, tmp, as_);
-        face_coef<R>(sch, de, fe, ae, tmp);
-        face_coef<R>(sch, dw, fw, tmp, aw);
-        face_coef<R>(sch, dt, ft, at, tmp);
-        face_coef<R>(sch, db, fb, tmp, ab);
-        vol = (R)volume_w(g, i, j, k);
-        apnot = rc * vol / delt;
-        R delf = fn - fs + fe - fw + ft - fb;
-        R cp0 = maxd(R(0), delf), cp1 = mind(R(0), delf);
-        su = -cp1 * w[c];
-        su += aij * (g.pressure[c - sk] - g.pressure[c]);
-        sp = -cp0;
+        q.ve = (i == nim2) ? vis_w : vis_w * viswe / ((R(1) - (R)fx[i]) * viswe + (R)fx[i] * vis_w);
+        q.vw = (i == 1) ? vis_w : vis_w * visww / ((R)fx[i - 1] * visww + (R(1) - (R)fx[i - 1]) * vis_w);
+        q.vt = vis[c];
+        q.vb = vis[c - sk];
+        q.dn = q.vn * awik * (R)g.dypsinv[j + 1];
+        q.ds = q.vs * awik * (R)g.dypsinv[j];
+        q.de = q.ve * awjk * (R)g.dxpwinv[i + 1];
+        q.dw = q.vw * awjk * (R)g.dxpwinv[i];
+        q.dt = q.vt * aij / (R)(zw[k + 1] - zw[k]);
+        q.db = q.vb * aij / (R)(zw[k] - zw[k - 1]);
+        q.a1 = awik; q.a2 = awjk; q.a3 = aij;
+        q.vol = (R)volume_w(g, i, j, k);
+        cn = c - sk;
+        flv = g.fracl[c] * (R(1) - fzm) + g.fracl[c - sk] * fzm;
+        R boufac = rc * (R)p.grav * (R)p.beta;
+        R tw = g.temp[c] * (R(1) - fzm) + g.temp[c - sk] * fzm;
+        q.bv = boufac * q.vol;
+        q.dtw = tw - (R)p.tsolid;
+    }
+    q.rc = rc;
+    q.apnot = rc * q.vol / delt;
+    q.term = (R)p.darcyKo * ((R(1) - flv) * (R(1) - flv)) / ((flv * flv * flv) + (R)kSmall);
+    q.flags = (flv > R(0) ? R(1) : R(0)) + (mind(g.temp[c], g.temp[cn]) <= (R)p.tsolid ? R(2) : R(0));
+}
+
+// One cell of the u/v/w equation (ivar 1..3) of the momentum box from its CellPre: the
+// coefficients, source, under-relaxation, the solid freeze and d = A/ap; returns
+// |residual| of the cell (calculateResiduals(1..3)).
+template <typename T, class LD>
+__device__ __forceinline__ double mom_cell_flow(const Params &p, const Fields<T> &g, const Status *st, int ivar, int i,
+                                                int j, int k, const CellPre<T> &e, CellEq<T> &q)
+{
+    using R = T;
+    const int nj = p.nj, nip = p.nip, nkm2 = p.nkm2;
+    const size_t sj = nip, sk = (size_t)nj * nip;
+    const int sch = p.scheme;
+    const LD u{g.uvel}, v{g.vvel}, w{g.wvel};
+    const double *xu = g.xu, *yv = g.yv, *zw = g.zw;
+    const size_t c = cidx(i, j, k, nj, nip);
+    R an, as_, ae, aw, at, ab, su, sp, tmp, areaD;
+    const R rc = e.rc, a1 = e.a1, a2 = e.a2, a3 = e.a3, vol = e.vol, apnot = e.apnot;
+    LD phi;
+    R urf, vn, vs, ue, uw, wt, wb;
+    if (ivar == 1) {
+        const R fxm = (R)g.fracx[i - 1];
+        vn = v[c + sj] * (R(1) - fxm) + v[c + sj - 1] * fxm;
+        vs = v[c] * (R(1) - fxm) + v[c - 1] * fxm;
+        ue = (u[c + 1] + u[c]) * R(0.5);
+        uw = (u[c - 1] + u[c]) * R(0.5);
+        wt = w[c + sk] * (R(1) - fxm) + w[c + sk - 1] * fxm;
+        wb = w[c] * (R(1) - fxm) + w[c - 1] * fxm;
+        phi = u; urf = (R)p.urfu; areaD = a2;
+    } else if (ivar == 2) {
+        const R fym = (R)g.fracy[j - 1];
+        vn = (v[c] + v[c + sj]) * R(0.5);
+        vs = (v[c] + v[c - sj]) * R(0.5);
+        ue = u[c + 1] * (R(1) - fym) + u[c + 1 - sj] * fym;
+        uw = u[c] * (R(1) - fym) + u[c - sj] * fym;
+        wt = w[c + sk] * (R(1) - fym) + w[c + sk - sj] * fym;
+        wb = w[c] * (R(1) - fym) + w[c - sj] * fym;
+        phi = v; urf = (R)p.urfv; areaD = a1;
+    } else {
+        const R fzm = (R)g.fracz[k - 1];
+        vn = v[c + sj] * (R(1) - fzm) + v[c + sj - sk] * fzm;
+        vs = v[c] * (R(1) - fzm) + v[c - sk] * fzm;
+        ue = u[c + 1] * (R(1) - fzm) + u[c + 1 - sk] * fzm;
+        uw = u[c] * (R(1) - fzm) + u[c - sk] * fzm;
+        wt = (w[c] + w[c + sk]) * R(0.5);
+        wb = (w[c] + w[c - sk]) * R(0.5);
+        phi = w; urf = (R)p.urfw; areaD = a3;
+    }
+    const R fn = vn * rc * a1, fs = vs * rc * a1, fe = ue * rc * a2, fw = uw * rc * a2;
+    const R ft = wt * rc * a3, fb = wb * rc * a3;
+    face_coef<R>(sch, e.dn, fn, an, tmp);
+    face_coef<R>(sch, e.ds, fs, tmp, as_);
+    face_coef<R>(sch, e.de, fe, ae, tmp);
+    face_coef<R>(sch, e.dw, fw, tmp, aw);
+    face_coef<R>(sch, e.dt, ft, at, tmp);
+    face_coef<R>(sch, e.db, fb, tmp, ab);
+    const R delf = fn - fs + fe - fw + ft - fb;
+    const R cp0 = maxd(R(0), delf), cp1 = mind(R(0), delf);
+    su = -cp1 * phi[c];
+    sp = -cp0;
+    if (ivar == 1) {
+        su += a2 * (g.pressure[c - 1] - g.pressure[c]);
+        su += apnot * g.unot[c];
+        R dudxp = (u[c + 1] - u[c]) / (R)(xu[i + 1] - xu[i]);
+        R dudxm = (u[c] - u[c - 1]) / (R)(xu[i] - xu[i - 1]);
+        su += (e.ve * dudxp - e.vw * dudxm) * a2;
+        R dvdxp = (v[c + sj] - v[c + sj - 1]) * (R)g.dxpwinv[i];
+        R dvdxm = (v[c] - v[c - 1]) * (R)g.dxpwinv[i];
+        su += (e.vn * dvdxp - e.vs * dvdxm) * a1;
+        R dwdxp = (w[c + sk] - w[c + sk - 1]) * (R)g.dxpwinv[i];
+        R dwdxm = (w[c] - w[c - 1]) * (R)g.dxpwinv[i];
+        su += (e.vt * dwdxp - e.vb * dwdxm) * a3;
+    } else if (ivar == 2) {
+        su += a1 * (g.pressure[c - sj] - g.pressure[c]);
+        su += apnot * g.vnot[c];
+        R dudyp = (u[c + 1] - u[c + 1 - sj]) * (R)g.dypsinv[j];
+        R dudym = (u[c] - u[c - sj]) * (R)g.dypsinv[j];
+        su += (e.ve * dudyp - e.vw * dudym) * a2;
+        R dvdyp = (v[c + sj] - v[c]) / (R)(yv[j + 1] - yv[j]);
+        R dvdym = (v[c] - v[c - sj]) / (R)(yv[j] - yv[j - 1]);
+        su += (e.vn * dvdyp - e.vs * dvdym) * a1;
+        R dwdyp = (w[c + sk] - w[c + sk - sj]) * (R)g.dypsinv[j];
+        R dwdym = (w[c] - w[c - sj]) * (R)g.dypsinv[j];
+        su += (e.vt * dwdyp - e.vb * dwdym) * a3;
+    } else {
+        su += a3 * (g.pressure[c - sk] - g.pressure[c]);
         su += apnot * g.wnot[c];
         R dudzp = (u[c + 1] - u[c + 1 - sk]) * (R)g.dzpbinv[k];
         R dudzm = (u[c] - u[c - sk]) * (R)g.dzpbinv[k];
-        su += (vise * dudzp - visw * dudzm) * awjk;
+        su += (e.ve * dudzp - e.vw * dudzm) * a2;
         R dvdzp = (v[c + sj] - v[c + sj - sk]) * (R)g.dzpbinv[k];
         R dvdzm = (v[c] - v[c - sk]) * (R)g.dzpbinv[k];
-        su += (visn * dvdzp - viss * dvdzm) * awik;
+        su += (e.vn * dvdzp - e.vs * dvdzm) * a1;
         R dwdzp = (w[c + sk] - w[c]) / (R)(zw[k + 1] - zw[k]);
         R dwdzm = (w[c] - w[c - sk]) / (R)(zw[k] - zw[k - 1]);
-        su += (vist * dwdzp - visb * dwdzm) * aij;
-        phi = w; cn = c - sk; urf = (R)p.urfw; areaD = aij;
-        flv = g.fracl[c] * (R(1) - fzm) + g.fracl[c - sk] * fzm;
+        su += (e.vt * dwdzp - e.vb * dwdzm) * a3;
     }
     // ---- calculateSource ----
-    if (flv > R(0)) {
-        R term = (R)p.darcyKo * ((R(1) - flv) * (R(1) - flv)) / ((flv * flv * flv) + (R)kSmall);
-        sp -= term * vol;
-        if (p.steady) {
-            R area = ivar == 1 ? (R)area_jk(p, g, j, k) : ivar == 2 ? (R)area_vjk(g, j, k)
-                                                                    : (R)area_wjk(g, j, k);
-            su += rc * (R)st->scanvel * area * (phi[c - 1] - phi[c]);
-        }
-        if (ivar == 3) {
-            R fzm = (R)fz[k - 1];
-            R boufac = rc * (R)p.grav * (R)p.beta;
-            R tw = g.temp[c] * (R(1) - fzm) + g.temp[c - sk] * fzm;
-            su += boufac * vol * (tw - (R)p.tsolid);
-        }
+    const int flags = (int)e.flags;
+    if (flags & 1) {
+        sp -= e.term * vol;
+        if (p.steady) su += rc * (R)st->scanvel * a2 * (phi[c - 1] - phi[c]);
+        if (ivar == 3) su += e.bv * e.dtw;
     }
     if (ivar != 3 && k == nkm2) {
         su += at * phi[c + sk];
@@ -355,7 +381,7 @@ __device__ __forceinline__ double mom_cell_eq(const Params &p, const Fields<T> &
     ap /= urf;
     su += (R(1) - urf) * ap * phi[c];
     dcoef *= urf;
-    if (mind(g.temp[c], g.temp[cn]) <= (R)p.tsolid) {
+    if (flags & 2) {
         su = R(0);
         an = as_ = ae = aw = at = ab = R(0);
         ap = (R)kLarge;
@@ -364,6 +390,14 @@ __device__ __forceinline__ double mom_cell_eq(const Params &p, const Fields<T> &
     q.pt = phi[c + sk]; q.pb = phi[c - sk]; q.pn = phi[c + sj]; q.ps = phi[c - sj];
     R r = an * q.pn + as_ * q.ps + ae * phi[c + 1] + aw * phi[c - 1] + at * q.pt + ab * q.pb + su - ap * phi[c];
     return fabs((double)r);
+}
+template <typename T, class LD>
+__device__ __forceinline__ double mom_cell_eq(const Params &p, const Fields<T> &g, const Status *st, int ivar, int i,
+                                              int j, int k, CellEq<T> &q)
+{
+    CellPre<T> e;
+    mom_cell_pre<T>(p, g, st, ivar, i, j, k, e);
+    return mom_cell_flow<T, LD>(p, g, st, ivar, i, j, k, e, q);
 }
 
 // The coefficients of cell c into the shared coefficient arrays.
@@ -1689,14 +1723,16 @@ mom_cluster_post_kernel(Params p, Fields<T> g, T *scratch, int smem_elems, const
 //     live, by st.async: the stores complete on the receiving line's mbarrier, so
 //     a value and the news of it travel together in one hop;
 //   * launches become cluster barriers, about 1 us each with the stores before
-//     them (14 of them), and the boundary values of the next equation and the
-//     residual sums run on the warps without a line while the others solve.
-// Measured (120x60x40 deck, box of 1600 cells, 98 lines on 16 CTAs): 52 us a chain
-// in FP32 and 90 in FP64, of which the eight passes take 4.2-5.6 us an equation and
-// the assembly 5.4-6.7 (FP32) and 11-15 (FP64), a serial stretch of divisions; the
-// step 4.78 -> 4.15 ms in FP32 and 6.92 -> 5.78 in FP64 (with fields read), the
-// reference's order on 61x31x21 cells 31.8 -> 18.1 ms.  L2 prefetches of the rows the
-// first assembly reads gained nothing (66.5 -> 68 us on the 400x200x100 deck).
+//     them (14 of them), and the boundary values of the next equation, the part of
+//     its coefficients that does not depend on the flow, and the residual sums run
+//     on the warps without a line while the others solve.
+// Measured (120x60x40 deck, box of 1600 cells, 98 lines on 16 CTAs): 47 us a chain in FP32
+// and 79 in FP64, of which the eight passes take 4.2-5.6 us an equation and the assembly
+// 3-5 (FP32) and 7-10 (FP64), a serial stretch of divisions; the chain in one piece of
+// assembly 52 and 90; the step (with fields read) 4.78 ms in FP32 and 6.92 in FP64 with the
+// multi-launch chain, 4.15 and 5.78 with this one, the reference's order on 61x31x21
+// cells 31.8 and 18.1 ms.  L2 prefetches of the rows the first assembly reads gained
+// nothing (66.5 -> 68 us on the 400x200x100 deck).
 // The arithmetic is that of the multi-launch chain operation for operation
 // (line_rhs, the scans of solve_line_regs, factor_cell; the residual sums are
 // formed from per-cell values in the order of its per-CTA partials), so both give
@@ -1996,18 +2032,51 @@ mom_chain_kernel(Params p, Fields<T> g, double *red, int nb_region, double *rcel
         f.k = k;
         mbar_init(reinterpret_cast<uint64_t *>(&f.bar));
     }
-    for (int q = t; q < b.n; q += nt) {
-        int i, j, k;
-        box_cell(b, q, i, j, k);
-        clean_cell<T>(p, g, i, j, k);
-    }
+    // Warps without a line.  Where there is one for every line they form what an equation
+    // needs besides the flow (CellPre) while the others do what leads up to it, and
+    // leave it in the half of the lines' shared memory that so few lines do not use.
+    const int idle = fits && lpc < nw ? nw - lpc : 0;
+    const bool ahead = idle >= lpc && lpc <= kChainLines / 2;
+    const bool helper = warp >= nw - idle;
+    T *pre = reinterpret_cast<T *>(lines + kChainLines / 2);
+    constexpr int kPre = sizeof(CellPre<T>) / sizeof(T);
+    static_assert(kPre * kChainCells * sizeof(T) <= sizeof(ChainLine<T>) * 2, "a line's CellPre fits two unused lines");
+    auto prepare = [&](int iv) {
+        for (int l = warp - (nw - idle); l < nloc; l += idle) {
+            int j, k;
+            if (!slot_line(first + l, j, k)) continue;
+#pragma unroll 1
+            for (int i = lane; i < n; i += 32) {
+                CellPre<T> e;
+                mom_cell_pre<T>(p, g, st, iv, i0 + i, j, k, e);
+                const T *v = reinterpret_cast<const T *>(&e);
+#pragma unroll
+                for (int q = 0; q < kPre; ++q) pre[((size_t)l * kPre + q) * kChainCells + i] = v[q];
+            }
+        }
+        __syncwarp();
+    };
     __syncthreads();
-    cluster_barrier();
+    if (ahead && helper) {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        prepare(1);
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    } else {
+        const int tc = ahead ? ((int)rank * lpc + warp) * 32 + lane : t, nc_ = ahead ? (int)nc * lpc * 32 : nt;
+        for (int q = tc; q < b.n; q += nc_) {
+            int i, j, k;
+            box_cell(b, q, i, j, k);
+            clean_cell<T>(p, g, i, j, k);
+        }
+        cluster_barrier();
+    }
     {
         int ntop;
         const int nbc = mom_bc_items(p, st, b, 1, ntop);
         double um = 0.0;
-        for (int q = t; q < nbc; q += nt) um = maxd(um, mom_bc_item<T, LD>(p, g, st, b, 1, q, ntop));
+        const int tc = ahead ? ((int)rank * lpc + warp) * 32 + lane : t, nc_ = ahead ? (int)nc * lpc * 32 : nt;
+        for (int q = tc; q < nbc && !(ahead && helper); q += nc_)
+            um = maxd(um, mom_bc_item<T, LD>(p, g, st, b, 1, q, ntop));
         um = cta_max(um, sh);
         if (threadIdx.x == 0) red[((size_t)4 * nb_region + rank) * R_NSLOTS + R_UMAX] = um;
     }
@@ -2018,18 +2087,19 @@ mom_chain_kernel(Params p, Fields<T> g, double *red, int nb_region, double *rcel
     const bool cells = b.n <= rcap;  // per-cell residuals kept (else per-CTA sums, in another order)
     const int nblk = cells ? (b.n + 255) / 256 : 0;
     // Work of equation `iv` beside its visits, spread over `nh` threads from `h`: the
-    // boundary values of the next equation, and the residual sums in the order of
-    // the multi-launch assemblies (blocks of 256 box cells: eight warp trees and a
-    // tree over them).  It needs every line's assembly of the equation done.
+    // boundary values of the next equation; with p', the residual sums of all four in
+    // the order of the multi-launch assemblies (blocks of 256 box cells: eight warp
+    // trees and a tree over them).  It needs every line's assembly of the equation done.
     auto beside = [&](int iv, int h, int nh) {
         if (iv <= 3) {
             int ntop;
             const int nbc = mom_bc_items(p, st, b, iv + 1, ntop);
             for (int q = h; q < nbc; q += nh) mom_bc_item<T, LD>(p, g, st, b, iv + 1, q, ntop);
+            __syncwarp();
+            return;
         }
-        __syncwarp();
-        for (int q = h >> 5; q < (iv == 4 ? 2 : 1) * nblk; q += nh >> 5) {
-            const int blk = q % nblk, e = iv - 1 + q / nblk;
+        for (int q = h >> 5; q < 5 * nblk; q += nh >> 5) {
+            const int e = q / nblk, blk = q - e * nblk;
             double x[8], y = 0.0;
 #pragma unroll
             for (int v = 0; v < 8; ++v) {
@@ -2043,15 +2113,11 @@ mom_chain_kernel(Params p, Fields<T> g, double *red, int nb_region, double *rcel
                 if (lane == v) y = x[v];
             y = warp_sum(y);
             if (lane == 0)
-                red[((size_t)(iv - 1) * nb_region + blk) * R_NSLOTS +
-                    (iv <= 3 ? R_MSUMD : e == 3 ? R_MRESORM : R_MDENOM)] = y;
+                red[((size_t)min(e, 3) * nb_region + blk) * R_NSLOTS +
+                    (e < 3 ? R_MSUMD : e == 3 ? R_MRESORM : R_MDENOM)] = y;
         }
         __syncwarp();
     };
-    // the warps without a line do that while the others visit theirs (the first CTAs
-    // of a box with fewer lines than warps have some); otherwise every warp does it
-    // after its visits
-    const int idle = fits && lpc < nw ? nw - lpc : 0;
 #pragma unroll 1
     for (int ivar = 1; ivar <= 4; ++ivar) {
         if (ivar == 4) pdl_release();
@@ -2080,7 +2146,15 @@ mom_chain_kernel(Params p, Fields<T> g, double *red, int nb_region, double *rcel
                 const size_t qc = (size_t)((k - k0) * J + j - j0) * n + i;  // box-cell order
                 double r, rd = 0.0;
                 if (ivar <= 3) {
-                    r = mom_cell_eq<T, LD>(p, g, st, ivar, i0 + i, j, k, q);
+                    CellPre<T> e;
+                    if (ahead) {
+                        T *v = reinterpret_cast<T *>(&e);
+#pragma unroll
+                        for (int q = 0; q < kPre; ++q) v[q] = pre[((size_t)l * kPre + q) * kChainCells + i];
+                    } else {
+                        mom_cell_pre<T>(p, g, st, ivar, i0 + i, j, k, e);
+                    }
+                    r = mom_cell_flow<T, LD>(p, g, st, ivar, i0 + i, j, k, e, q);
                     (ivar == 1 ? g.dux : ivar == 2 ? g.dvy : g.dwz)[c] = q.d;
                 } else {
                     r = 0.0;
@@ -2179,8 +2253,10 @@ mom_chain_kernel(Params p, Fields<T> g, double *red, int nb_region, double *rcel
             }
             __syncwarp();
             asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-            if (warp >= nw - idle)
+            if (helper) {
                 beside(ivar, ((int)rank * idle + warp - (nw - idle)) * 32 + lane, (int)nc * idle * 32);
+                if (ahead && ivar < 3) prepare(ivar + 1);
+            }
         } else {
             __syncwarp();
             asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
