@@ -288,9 +288,16 @@ __global__ void __launch_bounds__(256) block_correct_kernel(Params p, Fields<T> 
 // peak-temperature maximum (BoundCondManager.cpp:301) and the reductions of
 // calculateFluxes (BoundCondManager.cpp:778-843): boundary conduction fluxes,
 // heat accumulation and volumetric heat input.  H->T is evaluated in FP64.
+// Bound by issue and by the FP64 conversions in FP32 (176 instructions a cell, XU 38 %,
+// DRAM 32 %), by its divisions in FP64.  A warp that keeps to one chunk of the row, widths
+// loaded once, the peak in the bulk precision and no conversion of a fraction that did not
+// change: with the melt-pool step 88 -> 76 us on 400x200x100 cells, 178 -> 148 on
+// 600x300x120, 26 -> 25 on 163x81x50; FP64 400x200x100 120 -> 115.  Three CTAs a SM: with
+// four, some of the registers are spilled (80 us); five are as good on 400x200x100 but cost
+// 120x60x40 3 us.
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(256, 4) h2t_kernel(Params p, Fields<T> g, double *red)
+__global__ void __launch_bounds__(256, 3) h2t_kernel(Params p, Fields<T> g, double *red)
 {
     pdl_wait();
     const Status *st = g.st;
@@ -304,7 +311,8 @@ __global__ void __launch_bounds__(256, 4) h2t_kernel(Params p, Fields<T> g, doub
     constexpr bool kExact = sizeof(T) == sizeof(double);
     const double inv_acpl = 1.0 / p.acpl, inv_acpa = 1.0 / p.acpa,
                  inv_mush = 1.0 / (p.hlcal - p.hsmelt), inv_delt = 1.0 / delt;
-    double tmax = -INFINITY, accul = 0.0, heatvol = 0.0;
+    T tpeak = (T)-INFINITY;
+    double accul = 0.0, heatvol = 0.0;
     const size_t sj = nip, sk = (size_t)nj * nip;
     const int js = st->jstart, is0 = st->istart;
     const double ts = p.tsolid;
@@ -314,97 +322,109 @@ __global__ void __launch_bounds__(256, 4) h2t_kernel(Params p, Fields<T> g, doub
     // Work unit: a chunk of 32 V cells of one x-line, V = 16 bytes per element;
     // lane l holds the 16-byte vector of cells base = chunk start + V l (the pitch
     // nip is a multiple of 32, so a vector lies wholly inside or wholly past the
-    // padded row).  Chunk indices are 32-bit (the chunk count is bounded at
-    // context creation): a 64-bit division per chunk costs more than the
-    // chunk's enthalpy inversions.
+    // padded row).  A warp keeps to one chunk of the row, so that what depends on x
+    // alone is formed once, and steps over the rows (32-bit: their count is bounded
+    // at context creation; a 64-bit division costs more than a chunk's enthalpy
+    // inversions).
     constexpr int V = 16 / (int)sizeof(T);
     constexpr int RC = 32 * V;
     const unsigned cpr = ((unsigned)nip + RC - 1) / RC;  // chunks per row
-    const unsigned unj = (unsigned)nj;
-    const unsigned nchunks = (unsigned)nk * unj * cpr;
+    const unsigned unj = (unsigned)nj, nrows = (unsigned)nk * unj;
     const unsigned W = gridDim.x * (blockDim.x >> 5);
     const unsigned w0 = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const unsigned step = max(1u, W / cpr);  // warps a chunk of the row
     const double *dxw = g.dxpwinv, *dys = g.dypsinv, *dzb = g.dzpbinv;
-    for (unsigned q = w0; q < nchunks; q += W) {
-        const unsigned r = q / cpr;
-        const int base = (int)(q - r * cpr) * RC + V * lane;
-        const int k = (int)(r / unj), j = (int)(r - (unsigned)k * unj);
-        const bool inrow = base < nip;
-        const size_t c0 = (size_t)r * nip + (inrow ? base : 0);
-        T hv[V], hn[V], fln[V], rn[V], sv[V];
-        ld16(g.h + c0, hv); ld16(g.hnot + c0, hn); ld16(g.fraclnot + c0, fln);
-        ld16(g.rho_nxt + c0, rn);
-        // the volumetric source input is zero everywhere without a volumetric source
-        if (volsrc) ld16(g.sourceinput + c0, sv);
-        const bool rowint = !steady && j >= 1 && j <= njm2 && k >= 1 && k <= nkm2;
-        T tout[V], fout[V];
-        int cmaxl = INT_MAX, cminl = INT_MIN;  // beam-row length candidates of this lane
+    for (unsigned w = w0; w < cpr * step; w += W) {
+        const int base = (int)(w % cpr) * RC + V * lane;
+        const bool inrow = base < nip, whole = base + V <= ni;
+        double xw[V + 1];  // the cells' faces (their difference is taken where it is used, so
+                           // that a warp's first row is on its way before they are waited for)
 #pragma unroll
-        for (int v = 0; v < V; ++v) {
-            const int i = base + v;
-            tout[v] = fout[v] = T(0);
-            if (!inrow || i >= ni) continue;
-            const double h = (double)hv[v];
-            double fl, t;
-            if (h >= p.hlcal) {
-                fl = 1.0;
-                t = (kExact ? (h - p.hlcal) / p.acpl : (h - p.hlcal) * inv_acpl) + p.tliquid;
-            } else if (h <= p.hsmelt) {
-                fl = 0.0;
-                const double root = sqrt(p.acpb * p.acpb + 2 * p.acpa * h) - p.acpb;
-                t = kExact ? root / p.acpa : root * inv_acpa;
-            } else {
-                fl = kExact ? (h - p.hsmelt) / (p.hlcal - p.hsmelt) : (h - p.hsmelt) * inv_mush;
-                t = deltemp * fl + p.tsolid;
+        for (int v = 0; v <= V; ++v) xw[v] = g.xu[min(base + v, ni - 1)];
+        for (unsigned r = w / cpr; r < nrows; r += step) {
+            const int k = (int)(r / unj), j = (int)(r - (unsigned)k * unj);
+            const size_t c0 = (size_t)r * nip + (inrow ? base : 0);
+            T hv[V], hn[V], fln[V], rn[V], sv[V];
+            ld16(g.h + c0, hv); ld16(g.hnot + c0, hn); ld16(g.fraclnot + c0, fln);
+            ld16(g.rho_nxt + c0, rn);
+            // the volumetric source input is zero everywhere without a volumetric source
+            if (volsrc) ld16(g.sourceinput + c0, sv);
+            const bool rowint = !steady && j >= 1 && j <= njm2 && k >= 1 && k <= nkm2;
+            const double dy = rowint ? g.yv[j + 1] - g.yv[j] : 0.0, dz = rowint ? g.zw[k + 1] - g.zw[k] : 0.0;
+            T tout[V], fout[V];
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                tout[v] = fout[v] = T(0);
+                if (!inrow || (!whole && base + v >= ni)) continue;
+                const double h = (double)hv[v];
+                double t;
+                if (h >= p.hlcal) {
+                    fout[v] = T(1);
+                    t = (kExact ? (h - p.hlcal) / p.acpl : (h - p.hlcal) * inv_acpl) + p.tliquid;
+                } else if (h <= p.hsmelt) {
+                    const double root = sqrt(p.acpb * p.acpb + 2 * p.acpa * h) - p.acpb;
+                    t = kExact ? root / p.acpa : root * inv_acpa;
+                } else {
+                    const double fl = kExact ? (h - p.hsmelt) / (p.hlcal - p.hsmelt) : (h - p.hsmelt) * inv_mush;
+                    fout[v] = (T)fl;
+                    t = deltemp * fl + p.tsolid;
+                }
+                tout[v] = (T)t;
+                if (tout[v] > tpeak) tpeak = tout[v];
+                if (!rowint || base + v < 1 || base + v > nim2) continue;
+                double dh1 = h - (double)hn[v];
+                if (fout[v] != fln[v]) dh1 += ((double)fout[v] - (double)fln[v]) * p.hlatnt;
+                const double vol = (xw[v + 1] - xw[v]) * dy * dz;
+                accul += kExact ? vol * (double)rn[v] * dh1 / delt : vol * (double)rn[v] * dh1 * inv_delt;
+                if (volsrc) heatvol += (double)sv[v] * vol;
             }
-            fout[v] = (T)fl;
-            tout[v] = (T)t;
-            const double tt = (double)(T)t;
-            if (tt > tmax) tmax = tt;
-            // melt-pool scan candidates (BoundCondManager.cpp:318-417).  Most cells
-            // are solid, so each atomic is issued only when it can still change the
-            // value (candidates only move one way); the beam-row scalars are
-            // warp-reduced below.
-            if (j == js && k >= 1 && k <= nkm2 && tt < ts && k > *(volatile int *)&g.mp_kb[i])
-                atomicMax(&g.mp_kb[i], k);
-            if (k == nkm1) {
-                if (j >= js && j <= njm2 && tt < ts && j < *(volatile int *)&g.mp_jup[i])
-                    atomicMin(&g.mp_jup[i], j);
-                if (j >= 1 && j <= js && tt < ts && j > *(volatile int *)&g.mp_jdn[i])
-                    atomicMax(&g.mp_jdn[i], j);
-                if (j == js) {
-                    if (i >= is0 && i < nim1 && tt <= ts) cmaxl = min(cmaxl, i);
-                    if (i >= 1 && i <= is0 && tt < ts) cminl = max(cminl, i);
+            if (inrow) {
+                if (whole) {
+                    typename Vec16<T>::type w;
+                    memcpy(&w, tout, 16);
+                    *reinterpret_cast<typename Vec16<T>::type *>(g.temp + c0) = w;
+                    memcpy(&w, fout, 16);
+                    *reinterpret_cast<typename Vec16<T>::type *>(g.fracl + c0) = w;
+                } else {
+#pragma unroll
+                    for (int v = 0; v < V; ++v)
+                        if (base + v < ni) {
+                            g.temp[c0 + v] = tout[v];
+                            g.fracl[c0 + v] = fout[v];
+                        }
                 }
             }
-            if (!rowint || i < 1 || i > nim2) continue;
-            const double dh1 = h - (double)hn[v] + ((double)(T)fl - (double)fln[v]) * p.hlatnt;
-            const double vol = volume_p(p, g, i, j, k);
-            accul += kExact ? vol * (double)rn[v] * dh1 / delt : vol * (double)rn[v] * dh1 * inv_delt;
-            if (volsrc) heatvol += (double)sv[v] * vol;
-        }
-        if (inrow) {
-            if (base + V <= ni) {
-                typename Vec16<T>::type w;
-                memcpy(&w, tout, 16);
-                *reinterpret_cast<typename Vec16<T>::type *>(g.temp + c0) = w;
-                memcpy(&w, fout, 16);
-                *reinterpret_cast<typename Vec16<T>::type *>(g.fracl + c0) = w;
-            } else {
+            // melt-pool scan candidates (BoundCondManager.cpp:318-417), on the beam's
+            // plane and on the top plane.  Most cells are solid, so each atomic is
+            // issued only when it can still change the value (candidates only move one
+            // way); the beam-row scalars are warp-reduced.
+            if (k != nkm1 && (j != js || k < 1 || k > nkm2)) continue;
+            int cmaxl = INT_MAX, cminl = INT_MIN;  // beam-row length candidates of this lane
 #pragma unroll
-                for (int v = 0; v < V; ++v)
-                    if (base + v < ni) {
-                        g.temp[c0 + v] = tout[v];
-                        g.fracl[c0 + v] = fout[v];
+            for (int v = 0; v < V; ++v) {
+                const int i = base + v;
+                if (!inrow || i >= ni) continue;
+                const double tt = (double)tout[v];
+                if (j == js && k >= 1 && k <= nkm2 && tt < ts && k > *(volatile int *)&g.mp_kb[i])
+                    atomicMax(&g.mp_kb[i], k);
+                if (k == nkm1) {
+                    if (j >= js && j <= njm2 && tt < ts && j < *(volatile int *)&g.mp_jup[i])
+                        atomicMin(&g.mp_jup[i], j);
+                    if (j >= 1 && j <= js && tt < ts && j > *(volatile int *)&g.mp_jdn[i])
+                        atomicMax(&g.mp_jdn[i], j);
+                    if (j == js) {
+                        if (i >= is0 && i < nim1 && tt <= ts) cmaxl = min(cmaxl, i);
+                        if (i >= 1 && i <= is0 && tt < ts) cminl = max(cminl, i);
                     }
+                }
             }
-        }
-        if (k == nkm1 && j == js) {  // chunk-uniform: every lane takes part
-            const int wmin = __reduce_min_sync(0xffffffffu, cmaxl);
-            const int wmax = __reduce_max_sync(0xffffffffu, cminl);
-            if (lane == 0) {
-                if (wmin != INT_MAX) atomicMin(&g.st->mp_imax, wmin);
-                if (wmax != INT_MIN) atomicMax(&g.st->mp_imin, wmax);
+            if (k == nkm1 && j == js) {  // row-uniform: every lane takes part
+                const int wmin = __reduce_min_sync(0xffffffffu, cmaxl);
+                const int wmax = __reduce_max_sync(0xffffffffu, cminl);
+                if (lane == 0) {
+                    if (wmin != INT_MAX) atomicMin(&g.st->mp_imax, wmin);
+                    if (wmax != INT_MIN) atomicMax(&g.st->mp_imin, wmax);
+                }
             }
         }
     }
@@ -415,12 +435,13 @@ __global__ void __launch_bounds__(256, 4) h2t_kernel(Params p, Fields<T> g, doub
     double fw = 0.0, fe = 0.0, fb = 0.0, ft = 0.0, fs = 0.0, fn = 0.0;
     {
         const int I = nim2, J = njm2, K = nkm2;  // interior extents
-        const long long nx = (long long)J * K, ny = (long long)I * K, nz = (long long)I * J;
-        const long long nall = 2 * (nx + ny + nz);
-        const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-        const long long nthr = (long long)gridDim.x * blockDim.x;
-        for (long long q = tid; q < nall; q += nthr) {
-            long long r = q;
+        // 32-bit: twice the faces of any domain whose arrays fit the memory
+        const unsigned nx = (unsigned)J * K, ny = (unsigned)I * K, nz = (unsigned)I * J;
+        const unsigned nall = 2 * (nx + ny + nz);
+        const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x;
+        const unsigned nthr = gridDim.x * blockDim.x;
+        for (unsigned q = tid; q < nall; q += nthr) {
+            unsigned r = q;
             int face, a, b;  // face 0..5 = W E B T S N
             if (r < 2 * nx) { face = (int)(r / nx); r %= nx; a = (int)(r % J); b = (int)(r / J); }
             else if ((r -= 2 * nx) < 2 * nz) { face = 2 + (int)(r / nz); r %= nz; a = (int)(r % I); b = (int)(r / I); }
@@ -442,7 +463,7 @@ __global__ void __launch_bounds__(256, 4) h2t_kernel(Params p, Fields<T> g, doub
             }
         }
     }
-    double v[8] = {tmax, accul, heatvol, fw, fe, fb, ft, fs};
+    double v[8] = {(double)tpeak, accul, heatvol, fw, fe, fb, ft, fs};
     const int s[8] = {R_TPEAK, R_ACCUL, R_HEATVOL, R_FW, R_FE, R_FB, R_FT, R_FS};
     const bool m[8] = {true, false, false, false, false, false, false, false};
     block_reduce_store<8>(v, s, m, red, blockIdx.x);
