@@ -224,8 +224,10 @@ __global__ void __launch_bounds__(256) block_correct_kernel(Params p, Fields<T> 
                                                             int nblk_asm, int check_finite, int ivar)
 {
     pdl_enter();
-    extern __shared__ double sm[];  // 4 * nip
-    __shared__ double sh[8][33];
+    // 4 * nip; first the partial sums of the 8 rows of threads (rows of 1502 cells fit the
+    // 48 KB that need no opt-in because they share the space)
+    extern __shared__ double sm[];
+    double (*sh)[33] = reinterpret_cast<double (*)[33]>(sm);
     __shared__ double grp[2][32];
     __shared__ int last;
     const int nip = p.nip, nim2 = p.nim2;
@@ -842,7 +844,8 @@ template <typename T> void launch_energy_bc(Inst<T> &I)
 }
 template <typename T> void launch_block_correct(Inst<T> &I, int ivar)
 {
-    launch_k(I.pdl, block_correct_kernel<T>, dim3(I.p.nip / 32, 4), dim3(32, 8), 4 * I.p.nip * sizeof(double), I.stream,
+    launch_k(I.pdl, block_correct_kernel<T>, dim3(I.p.nip / 32, 4), dim3(32, 8),
+             std::max(4 * I.p.nip, 8 * 33) * sizeof(double), I.stream,
              I.p, I.g, I.red_asm, I.nb_asm, I.check_finite, ivar);
 }
 // Field read-out: the padded [k][j][nip] array widened to FP64 and packed to

@@ -20,7 +20,8 @@ def _deck(tmp, nx, ny, nz):
 # small launch has warps for, and boxes of three planes
 @pytest.mark.parametrize("prec", [0, 1])
 @pytest.mark.parametrize("nx,ny,nz", [(5, 4, 3), (62, 9, 6), (64, 8, 5), (126, 6, 5), (128, 7, 4), (254, 5, 4),
-                                      (257, 30, 9), (700, 4, 3), (1400, 3, 3), (90, 120, 3)])
+                                      (257, 30, 9), (700, 4, 3), (1400, 3, 3),
+                                      (1502, 3, 3), (90, 120, 3)])
 def test_inversion_of_every_node(prec, nx, ny, nz, tmp_path):
     import amcfd
     d, path = _deck(tmp_path, nx, ny, nz)
