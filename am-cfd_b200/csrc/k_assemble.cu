@@ -117,6 +117,14 @@ template <typename R> struct AsmConst {
 // FP32 (64 registers, some spilled in the long form) hide more of the planes' latency
 // where there are CTAs for them (225 -> 208 on 400x200x100) and cost the spills where
 // there are not (32.7 -> 36.5 on 120x60x40).
+//
+// Of the short form, a ninth is choices between a face inside and one on the boundary, which
+// a warp away from it need not make (INNER): with unsigned ring indices a step's iteration
+// 652 -> 645 us on 400x200x100 cells, FP64 1096 -> 1074, 600x300x120 1349 -> 1332.  Not
+// under defect correction, nor on rows of fewer than six tiles, where a third of the
+// warps and more are at the boundary: there the instructions of a third form cost more
+// (200x100x60 DC 295 -> 301, FP64 120x60x40 229.0 -> 229.8).
+constexpr unsigned kInnerTiles = 6;
 template <typename T, int SCH, bool DC, bool CALM, int OCC>
 __global__ void __launch_bounds__(256, OCC)
 energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant__ AsmMaps mp, DcBuf dco,
@@ -155,10 +163,10 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
     // ---- copy pipeline ----
     // Slots are filled in plane order (ring A from plane kb-1, ring B from kb),
     // so the n-th fill of a slot completes its barrier's phase of parity n & 1.
-    auto slotA = [&](int q) { return (q - kb + 1) % B::SA; };
-    auto parA = [&](int q) { return (uint32_t)(((q - kb + 1) / B::SA) & 1); };
-    auto slotB = [&](int q) { return (q - kb) % B::SB; };
-    auto parB = [&](int q) { return (uint32_t)(((q - kb) / B::SB) & 1); };
+    auto slotA = [&](int q) { return (unsigned)(q - kb + 1) % B::SA; };
+    auto parA = [&](int q) { return (unsigned)(q - kb + 1) / B::SA & 1u; };
+    auto slotB = [&](int q) { return (unsigned)(q - kb) % B::SB; };
+    auto parB = [&](int q) { return (unsigned)(q - kb) / B::SB & 1u; };
     auto issueA = [&](int q) {
         const int s = slotA(q);
         T *dst = bufA + s * B::NA * FE;
@@ -234,6 +242,7 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
     // bit with the reference): one reciprocal per face instead of two divisions,
     // and the divisions by per-launch constants as multiplications
     constexpr bool FAST = kF32 || DC;
+    constexpr bool kInner = CALM && !DC;  // the form without boundary faces (INNER below)
     const R fdx = (R)dx, fdy = (R)dy;
     const R inv_delt = (R)(1.0 / delt);
     // per-launch constants in the bulk precision stay in the kernel's parameters (as
@@ -241,6 +250,8 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
     const R &inv_acpl = cst.inv_acpl, &inv_urfh = cst.inv_urfh, &thla = cst.thla, &thlb = cst.thlb, &acpl = cst.acpl,
             &thsa = cst.thsa, &thsb = cst.thsb, &thsc = cst.thsc, &acpa = cst.acpa, &acpb = cst.acpb,
             &tliq = cst.tliq, &tsol = cst.tsol, &denl = cst.denl, &dens = cst.dens, &visc = cst.visc;
+    const bool inner = kInner && gridDim.x >= kInnerTiles &&
+                       __all_sync(0xffffffffu, !colint || (i > 1 && i < nim2 && j > 1 && j < njm2));
     double sumd = 0.0, sumh = 0.0;
     double bl = 0.0, blp = 0.0, blm = 0.0, blc = 0.0;
     const int o = (ty + 1) * BX + tx + OX;  // this thread's cell inside a box
@@ -299,8 +310,9 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
             // warp are zero, so no face carries a mass flux: each coefficient is the face's
             // conductance (the scheme's A(0) = 1 exactly) and the convected latent heat is
             // nothing -- the same numbers without forming them.
-            auto interior = [&](auto still_c) {
-                constexpr bool STILL = decltype(still_c)::value;
+            // INNER: no cell of the warp has a face on the boundary either.
+            auto interior = [&](auto still_c, auto inner_c) {
+                constexpr bool STILL = decltype(still_c)::value, INNER = decltype(inner_c)::value;
                 const int kl = k - kb;
                 const double dz = pl_dz[kl];
                 const R fdz = pl_m[4][kl];
@@ -319,13 +331,13 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
                 {
                     const R fn = STILL ? R(0) : Ac[FA_R * FE + BX] * v_n * aik;
                     if constexpr (FAST) {
-                        const bool bnd = j == njm2;
+                        const bool bnd = !INNER && j == njm2;
                         const R num = bnd ? dcc * aik * dyp_p : dcc * d_nn * aik * dyp_p;
                         const R den = bnd ? R(1) : (R(1) - fy_j) * d_nn + fy_j * dcc;
                         face_fast<R, STILL>(sch, num, den, fn, an, tmp);
                     } else {
                         R dn;
-                        if (j == njm2) {
+                        if (!INNER && j == njm2) {
                             dn = dcc * aik * dyp_p;
                         } else {
                             R difn = bdiv(dcc * d_nn, (R(1) - fy_j) * d_nn + fy_j * dcc);
@@ -338,13 +350,13 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
                 {
                     const R fs = STILL ? R(0) : rhc * v_c * aik;
                     if constexpr (FAST) {
-                        const bool bnd = j == 1;
+                        const bool bnd = !INNER && j == 1;
                         const R num = bnd ? dcc * aik * dyp_j : d_s * dcc * aik * dyp_j;
                         const R den = bnd ? R(1) : (R(1) - fy_m) * dcc + fy_m * d_s;
                         face_fast<R, STILL>(sch, num, den, fs, tmp, as_);
                     } else {
                         R ds;
-                        if (j == 1) {
+                        if (!INNER && j == 1) {
                             ds = dcc * aik * dyp_j;
                         } else {
                             R difs = bdiv(d_s * dcc, (R(1) - fy_m) * dcc + fy_m * d_s);
@@ -357,13 +369,13 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
                 {
                     const R fe = STILL ? R(0) : Ac[FA_R * FE + 1] * u_e * ajk;
                     if constexpr (FAST) {
-                        const bool bnd = i == nim2;
+                        const bool bnd = !INNER && i == nim2;
                         const R num = bnd ? dcc * ajk * dxp_p : dcc * d_e * ajk * dxp_p;
                         const R den = bnd ? R(1) : (R(1) - fx_i) * d_e + fx_i * dcc;
                         face_fast<R, STILL>(sch, num, den, fe, ae, tmp);
                     } else {
                         R de;
-                        if (i == nim2) {
+                        if (!INNER && i == nim2) {
                             de = dcc * ajk * dxp_p;
                         } else {
                             R dife = bdiv(dcc * d_e, (R(1) - fx_i) * d_e + fx_i * dcc);
@@ -376,13 +388,13 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
                 {
                     const R fw = STILL ? R(0) : rhc * u_c * ajk;
                     if constexpr (FAST) {
-                        const bool bnd = i == 1;
+                        const bool bnd = !INNER && i == 1;
                         const R num = bnd ? dcc * ajk * dxp_i : d_w * dcc * ajk * dxp_i;
                         const R den = bnd ? R(1) : (R(1) - fx_m) * dcc + fx_m * d_w;
                         face_fast<R, STILL>(sch, num, den, fw, tmp, aw);
                     } else {
                         R dw;
-                        if (i == 1) {
+                        if (!INNER && i == 1) {
                             dw = dcc * ajk * dxp_i;
                         } else {
                             R difw = bdiv(d_w * dcc, (R(1) - fx_m) * dcc + fx_m * d_w);
@@ -395,13 +407,13 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
                 {
                     const R ft = STILL ? R(0) : Ap[FA_R * FE] * w_p * aij;
                     if constexpr (FAST) {
-                        const bool bnd = k == nkm2;
+                        const bool bnd = !INNER && k == nkm2;
                         const R num = bnd ? dcc * aij * dzp_p : dcc * d_p * aij * dzp_p;
                         const R den = bnd ? R(1) : (R(1) - fz_k) * d_p + fz_k * dcc;
                         face_fast<R, STILL>(sch, num, den, ft, at, ab_up);
                     } else {
                         R dt;
-                        if (k == nkm2) {
+                        if (!INNER && k == nkm2) {
                             dt = dcc * aij * dzp_p;
                         } else {
                             R dift = bdiv(dcc * d_p, (R(1) - fz_k) * d_p + fz_k * dcc);
@@ -418,13 +430,13 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
                 } else {
                     const R fb = STILL ? R(0) : rhc * w_c * aij;
                     if constexpr (FAST) {
-                        const bool bnd = k == 1;
+                        const bool bnd = !INNER && k == 1;
                         const R num = bnd ? dcc * aij * dzp_k : d_m * dcc * aij * dzp_k;
                         const R den = bnd ? R(1) : (R(1) - fz_m) * dcc + fz_m * d_m;
                         face_fast<R, STILL>(sch, num, den, fb, tmp, ab);
                     } else {
                         R db;
-                        if (k == 1) {
+                        if (!INNER && k == 1) {
                             db = dcc * aij * dzp_k;
                         } else {
                             R difb = bdiv(d_m * dcc, (R(1) - fz_m) * dcc + fz_m * d_m);
@@ -472,12 +484,12 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
                 const R hjp = Ac[FA_H * FE + BX], hjm = Ac[FA_H * FE - BX], hip = Ac[FA_H * FE + 1],
                         him = Ac[FA_H * FE - 1], hkp = Ap[FA_H * FE], hkm = Am[FA_H * FE];
                 // boundary folds, in the reference's order: k, j, i
-                if (k == 1) { su += ab * hkm; sp -= ab; ab = R(0); }
-                if (k == nkm2) { su += at * hkp; sp -= at; at = R(0); }
-                if (j == 1) { su += as_ * hjm; sp -= as_; as_ = R(0); }
-                if (j == njm2) { su += an * hjp; sp -= an; an = R(0); }
-                if (i == 1) { su += aw * him; sp -= aw; aw = R(0); }
-                if (i == nim2) { su += ae * hip; sp -= ae; ae = R(0); }
+                if (!INNER && k == 1) { su += ab * hkm; sp -= ab; ab = R(0); }
+                if (!INNER && k == nkm2) { su += at * hkp; sp -= at; at = R(0); }
+                if (!INNER && j == 1) { su += as_ * hjm; sp -= as_; as_ = R(0); }
+                if (!INNER && j == njm2) { su += an * hjp; sp -= an; an = R(0); }
+                if (!INNER && i == 1) { su += aw * him; sp -= aw; aw = R(0); }
+                if (!INNER && i == nim2) { su += ae * hip; sp -= ae; ae = R(0); }
                 R ap;
                 if constexpr (kF32)  // fused in both forms of a cell, so that they give the same bits
                     ap = fused(densbydt, vol, an + as_ + ae + aw + at + ab) - sp;
@@ -515,10 +527,12 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
                 blm += (double)aw;
             };
             if (cell) {
-                if (CALM && still)
-                    interior(std::bool_constant<CALM>{});
+                if (kInner && still && inner && k > 1 && k < nkm2)
+                    interior(std::bool_constant<CALM>{}, std::bool_constant<kInner>{});
+                else if (CALM && still)
+                    interior(std::bool_constant<CALM>{}, std::false_type{});
                 else
-                    interior(std::false_type{});
+                    interior(std::false_type{}, std::false_type{});
             }
         }
         // this warp is done with planes k-1 (ring A) and k (ring B); the last warp
@@ -527,7 +541,7 @@ energy_assemble_kernel(Params p, Fields<T> g, double *red, const __grid_constant
         __syncwarp();
         if (lane == 0) {
             __threadfence_block();
-            const int r = k - kb;
+            const unsigned r = (unsigned)(k - kb);
             const uint32_t n = atomicAdd(&done_cnt[r % kAsmCounters], 1u);
             if (n == (uint32_t)(kAsmWarps * (r / kAsmCounters + 1) - 1)) {
                 __threadfence_block();

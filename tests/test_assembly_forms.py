@@ -5,7 +5,8 @@ A warp whose cells see no flow takes a shorter form of the same cell; which
 instantiation runs follows from the number of CTAs, which the planes per CTA
 (asm_kseg) set.  From one state -- a melt pool with flow in a solid, still plate --
 every shape must give the same coefficients, sources and properties, bit for bit: the
-short form skips operations whose result is exact (A(0) = 1, + 0), nothing else.
+short form skips operations whose result is exact (A(0) = 1, + 0), nothing else, and where
+rows have six tiles and more a warp away from the boundary skips its choices too.
 FP64 compares the planes that begin no segment in either shape: a segment's first plane
 forms its bottom face afresh instead of carrying it from the plane below, in an
 expression that FP64 may round differently.
@@ -21,10 +22,13 @@ OUT = ("an", "as", "ae", "aw", "at", "ab", "ap", "su", "diff_next", "rho_next", 
 
 
 # 70x30x20: 24 CTAs at 16 planes, 72 at 4 (at most one a SM: the long form only);
-# 120x60x40: 96 and 352; 201x91x61: 336 and 1344 (FP32: four CTAs a SM)
+# 120x60x40: 96 and 352; 201x91x61: 336 and 1344 (FP32: four CTAs a SM); 160x38x20 and
+# 190x38x20 (rows of six tiles, the last one short and whole): 60 and 180, the long form
+# against the short one without boundary faces
 @pytest.mark.parametrize("prec", [0, 1, 2])
 @pytest.mark.parametrize("scheme", ["power_law", "upwind"])
-@pytest.mark.parametrize("nx,ny,nz", [(70, 30, 20), (120, 60, 40), (201, 91, 61)])
+@pytest.mark.parametrize("nx,ny,nz", [(70, 30, 20), (120, 60, 40), (160, 38, 20), (190, 38, 20),
+                                      (201, 91, 61)])
 def test_launch_shapes_give_the_same_coefficients(prec, scheme, nx, ny, nz, tmp_path):
     import amcfd
     import amcfd_decks as D
