@@ -584,7 +584,7 @@ __global__ void sweep_rb_kernel(Params p, Fields<T> g, T *phi, int color)
 // write; vectors past the end of the padded row read its first vector and are
 // masked.
 // FACTOR (the first pass of each colour): the line's factorisation is formed in
-// the same rounds from ap, aw, ae, as factor_rounds_kernel forms it, and
+// the same rounds from ap, aw, ae, exactly as factor_rounds_kernel forms it, and
 // stored for the later passes.  With `correct` (the first colour's first pass)
 // the block correction phi += delphi, which the factorisation kernel would have
 // stored into every interior line, is added to the neighbour values read from
@@ -595,6 +595,9 @@ __global__ void sweep_rb_kernel(Params p, Fields<T> g, T *phi, int color)
 // neighbour values are delphi on interior lines and zero on boundary lines,
 // and nothing is read from phi for them.
 // ---------------------------------------------------------------------------
+template <typename T>
+__device__ __forceinline__ void mat_rescale(T &a, T &b, T &c, T &d);
+
 // 16-byte vector load; CG: through L2 only (rows that other SMs write while the
 // kernel runs: the pipelined sweep's neighbour values and factorisation rows).
 template <bool CG, typename T>
@@ -610,15 +613,9 @@ __device__ __forceinline__ void ld16x(const T *ptr, T (&o)[16 / sizeof(T)])
 
 // The factorisation of one round of a line (V cells a lane from cell `base`): on
 // entry wc, wi, wp hold aw, ap, ae; on return cf, iden, pr (zero outside i0..i1).
-// carry_pr is pr of the cell before the round, then of its last.  pr follows the
-// projective map x -> ae / (ap - aw x), the matrix [[0, ae], [-aw, ap]]; the matrices of
-// the lanes below, chained by a warp scan, give a lane its entry value.  A map is
-// unchanged by a factor of its matrix, so every product is divided by its last entry
-// (a pivot: not zero where the line's systems have any), which is then one and need
-// neither be sent nor multiplied by.  A pipelined solve of 400x200x100 cells: 290 us,
-// 516 in FP64; with all four entries sent and divided by their largest, 294 and 535.
-// (Powers of two instead of the divide: 278 and 502, but pr's error against 64 bits was
-// 1 to 40 % larger; a factor of exactly one rounds nothing.)
+// carry_pr is pr of the cell before the round, then of its last.  The matrices
+// [[0, ae], [-aw, ap]] of the lanes below, chained by a warp scan, give a lane its
+// entry value (see factor_rounds_kernel).
 template <typename T>
 __device__ __forceinline__ void factor_round(T (&wc)[16 / sizeof(T)], T (&wi)[16 / sizeof(T)], T (&wp)[16 / sizeof(T)],
                                              int base, int i0, int i1, T &carry_pr)
@@ -635,22 +632,22 @@ __device__ __forceinline__ void factor_round(T (&wc)[16 / sizeof(T)], T (&wi)[16
             m00 = n00; m01 = n01; m10 = n10; m11 = n11;
         }
     }
-    T sc = T(1) / m11;
-    m00 *= sc; m01 *= sc; m10 *= sc;
+    mat_rescale(m00, m01, m10, m11);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const T b00 = __shfl_up_sync(full, m00, o), b01 = __shfl_up_sync(full, m01, o);
-        const T b10 = __shfl_up_sync(full, m10, o);
+        const T b10 = __shfl_up_sync(full, m10, o), b11 = __shfl_up_sync(full, m11, o);
         if (lane >= o) {  // own * lower
-            sc = T(1) / (m10 * b01 + T(1));
-            const T n00 = m00 * b00 + m01 * b10, n01 = m00 * b01 + m01, n10 = m10 * b00 + b10;
-            m00 = n00 * sc; m01 = n01 * sc; m10 = n10 * sc;
+            const T n00 = m00 * b00 + m01 * b10, n01 = m00 * b01 + m01 * b11;
+            const T n10 = m10 * b00 + m11 * b10, n11 = m10 * b01 + m11 * b11;
+            m00 = n00; m01 = n01; m10 = n10; m11 = n11;
+            mat_rescale(m00, m01, m10, m11);
         }
     }
     const T e00 = __shfl_up_sync(full, m00, 1), e01 = __shfl_up_sync(full, m01, 1);
-    const T e10 = __shfl_up_sync(full, m10, 1);
+    const T e10 = __shfl_up_sync(full, m10, 1), e11 = __shfl_up_sync(full, m11, 1);
     T x = carry_pr;
-    if (lane > 0) x = (e00 * carry_pr + e01) / (e10 * carry_pr + T(1));
+    if (lane > 0) x = (e00 * carry_pr + e01) / (e10 * carry_pr + e11);
 #pragma unroll
     for (int v = 0; v < V; ++v) {
         if (base + v >= i0 && base + v <= i1) {
@@ -1312,8 +1309,22 @@ sweep_resident_kernel(Params p, Fields<T> g, T *phi, int correct, int spc, int n
 // Whole-domain factorisation in the same 16-byte-vector rounds (one warp per
 // line): den_i = ap_i - aw_i pr_{i-1}, pr_i = ae_i/den_i, cf_i = aw_i/den_i,
 // iden_i = 1/den_i from pr_{i0-1} = 0, and phi += delphi (the block correction).
-// factor_round forms them.
+// pr follows the projective map x -> ae/(ap - aw x), i.e. the 2x2 matrix
+// [[0, ae], [-aw, ap]]: each lane multiplies the matrices of its cells, a warp
+// scan (rescaled as it goes; the map ignores scale) gives each lane the product
+// of the lanes below, applied to the carried pr of the previous round it is
+// the lane's entry value, and the lane then runs the recurrence itself.
 // ---------------------------------------------------------------------------
+template <typename T>
+__device__ __forceinline__ void mat_rescale(T &a, T &b, T &c, T &d)
+{
+    const T mx = fmax(fmax(fabs(a), fabs(b)), fmax(fabs(c), fabs(d)));
+    if (mx > T(0)) {
+        const T s = T(1) / mx;
+        a *= s; b *= s; c *= s; d *= s;
+    }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(128) factor_rounds_kernel(Params p, Fields<T> g, T *phi)
 {
@@ -1324,6 +1335,7 @@ __global__ void __launch_bounds__(128) factor_rounds_kernel(Params p, Fields<T> 
     const int J = p.njm2, K = p.nkm2;
     if (J <= 0 || K <= 0 || i1 < i0) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+    const unsigned full = 0xffffffffu;
     const int ib = i0 & ~31;
     const int R = (i1 - ib) / RC + 1;
     const int nj = p.nj, nip = p.nip, nl = J * K;
@@ -1335,29 +1347,67 @@ __global__ void __launch_bounds__(128) factor_rounds_kernel(Params p, Fields<T> 
             const int base = ib + RC * m + V * lane;
             const bool inrow = base + V <= nip;
             const size_t c = row + (inrow ? base : 0);
-            T wi[V], wc[V], wp[V], ph[V];
-            ld16(g.ap + c, wi); ld16(g.aw + c, wc); ld16(g.ae + c, wp); ld16(phi + c, ph);
-            factor_round<T>(wc, wi, wp, base, i0, i1, carry);
+            T ap[V], aw[V], ae[V], ph[V];
+            ld16(g.ap + c, ap); ld16(g.aw + c, aw); ld16(g.ae + c, ae); ld16(phi + c, ph);
             bool ok[V];
+            // product of this lane's matrices, last cell leftmost
+            T m00 = T(1), m01 = T(0), m10 = T(0), m11 = T(1);
 #pragma unroll
             for (int v = 0; v < V; ++v) {
                 ok[v] = base + v >= i0 && base + v <= i1;
-                if (ok[v]) ph[v] = ph[v] + (T)g.delphi[base + v];
+                if (ok[v]) {  // [[0, ae], [-aw, ap]] * M
+                    const T n00 = ae[v] * m10, n01 = ae[v] * m11;
+                    const T n10 = -aw[v] * m00 + ap[v] * m10, n11 = -aw[v] * m01 + ap[v] * m11;
+                    m00 = n00; m01 = n01; m10 = n10; m11 = n11;
+                }
             }
+            mat_rescale(m00, m01, m10, m11);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const T b00 = __shfl_up_sync(full, m00, o), b01 = __shfl_up_sync(full, m01, o);
+                const T b10 = __shfl_up_sync(full, m10, o), b11 = __shfl_up_sync(full, m11, o);
+                if (lane >= o) {  // own * lower
+                    const T n00 = m00 * b00 + m01 * b10, n01 = m00 * b01 + m01 * b11;
+                    const T n10 = m10 * b00 + m11 * b10, n11 = m10 * b01 + m11 * b11;
+                    m00 = n00; m01 = n01; m10 = n10; m11 = n11;
+                    mat_rescale(m00, m01, m10, m11);
+                }
+            }
+            // exclusive product applied to the carried pr
+            T e00 = __shfl_up_sync(full, m00, 1), e01 = __shfl_up_sync(full, m01, 1);
+            T e10 = __shfl_up_sync(full, m10, 1), e11 = __shfl_up_sync(full, m11, 1);
+            T x = carry;
+            if (lane > 0) x = (e00 * carry + e01) / (e10 * carry + e11);
+            T pr[V], cf[V], id[V];
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                if (ok[v]) {
+                    const T den = ap[v] - aw[v] * x;
+                    const T idv = T(1) / den;
+                    pr[v] = ae[v] * idv;
+                    cf[v] = aw[v] * idv;
+                    id[v] = idv;
+                    x = pr[v];
+                    ph[v] = ph[v] + (T)g.delphi[base + v];
+                } else {
+                    pr[v] = cf[v] = id[v] = T(0);
+                }
+            }
+            carry = __shfl_sync(full, x, 31);
             bool all = true;
 #pragma unroll
             for (int v = 0; v < V; ++v) all = all && ok[v];
             if (all) {
                 typename Vec16<T>::type w;
-                memcpy(&w, wp, 16); *reinterpret_cast<typename Vec16<T>::type *>(g.pr + c) = w;
-                memcpy(&w, wc, 16); *reinterpret_cast<typename Vec16<T>::type *>(g.cf + c) = w;
-                memcpy(&w, wi, 16); *reinterpret_cast<typename Vec16<T>::type *>(g.iden + c) = w;
+                memcpy(&w, pr, 16); *reinterpret_cast<typename Vec16<T>::type *>(g.pr + c) = w;
+                memcpy(&w, cf, 16); *reinterpret_cast<typename Vec16<T>::type *>(g.cf + c) = w;
+                memcpy(&w, id, 16); *reinterpret_cast<typename Vec16<T>::type *>(g.iden + c) = w;
                 memcpy(&w, ph, 16); *reinterpret_cast<typename Vec16<T>::type *>(phi + c) = w;
             } else {
 #pragma unroll
                 for (int v = 0; v < V; ++v)
                     if (ok[v]) {
-                        g.pr[c + v] = wp[v]; g.cf[c + v] = wc[v]; g.iden[c + v] = wi[v]; phi[c + v] = ph[v];
+                        g.pr[c + v] = pr[v]; g.cf[c + v] = cf[v]; g.iden[c + v] = id[v]; phi[c + v] = ph[v];
                     }
             }
         }
