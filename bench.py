@@ -616,11 +616,11 @@ def main():
                 "config": dict(cfg_desc, precision=args.precision, order=args.order, graphs=args.graphs,
                                outer_loop="host" if args.host_loop or not args.graphs else "device",
                                momentum=("grid" if args.no_small_box else "one-CTA below its capacity, else grid"
-                                         if args.small_box else "cooperative box solve"
-                                         " (one-CTA chain only where that is unavailable)")
+                                         if args.small_box else "one cluster launch for the chain"
+                                         " (cooperative box solve where its lines do not fit)")
                                + (", serial launches" if args.serial_launch else ""),
                                sweeps="a launch per pass" if args.pass_launch or args.serial_launch
-                               else "the 8 passes of a solve in one pipelined launch",
+                               else "the 8 passes of a solve in one launch",
                                parallelism=f"replicas{world}"),
                 "cell_iters_per_s": cips, "outer_iters": iters, "gpu_launches": launches,
                 "e2e": e2e, "roofline": roofline, "cpu_baseline": cpu, "clocks": ck,

@@ -160,8 +160,8 @@ typedef struct amcfd_options {
                             test convergence on the host (0: one graph per step, the
                             iterations chained on the device) */
     int wait_polls;      /* polls (about 64 ns each) a warp of a line sweep (the exact-order
-                            wavefront, the pipelined red-black passes, the cooperative
-                            momentum-box solve) waits for a neighbouring line before the step fails with
+                            sweep, the red-black passes of a solve in one launch, the
+                            momentum launches) waits for a neighbouring line before the step fails with
                             AMCFD_E_TIMEOUT; 0 = the default 2^24 (about one second).  The
                             reference has no such wait (its sweeps are sequential). */
     int autotune;        /* 1: at creation, time the candidate launch shapes of the energy
@@ -190,9 +190,9 @@ typedef struct amcfd_options {
                             them every pass) */
     int pass_launch;     /* 1: the whole-domain red-black line sweeps (enthalpy, species,
                             the defect correction) take one launch per colour pass; 0: the
-                            eight passes of a solve run in one launch, pipelined along k so
-                            that later passes find a plane's coefficient rows in L2 (the
-                            same bits: each line still reads its neighbours after exactly
+                            eight passes of a solve run in one launch, each line kept by a
+                            warp where the domain is small enough for it, pipelined along k
+                            otherwise (the same bits: each line still reads its neighbours after exactly
                             the passes the per-pass order gives it).  serial_launch = 1
                             implies 1. */
 } amcfd_options;
