@@ -575,7 +575,7 @@ __global__ void sweep_rb_kernel(Params p, Fields<T> g, T *phi, int color)
 //             carried from the round before (qr_{i0-1} = phi_{i0-1}), and the
 //             lane then runs its cells to get qr; qr and pr go to a per-warp
 //             buffer, by 16-byte vectors (by elements, four and two ways into a bank,
-//             a pipelined solve of 400x200x100 cells took 301 us against 294);
+//             a pipelined solve of 400x200x100 cells took 301 us against 291);
 //   backward: rounds in reverse, the maps x -> pr_i x + qr_i likewise with a
 //             suffix scan, applied to phi carried from the round after
 //             (phi_{i1+1} fixed); phi is stored.
