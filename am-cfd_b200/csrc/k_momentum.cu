@@ -1749,8 +1749,12 @@ mom_cluster_post_kernel(Params p, Fields<T> g, T *scratch, int smem_elems, const
 // of two visits never share an mbarrier phase.  A warp with two lines runs
 // their visits in the order of the pass (exact order: of the wave
 // t = 3m + (j-j0) + 2s of k_linesolve.cu), which every dependency precedes.
-// A wait that runs out (wait_polls) records AMCFD_E_TIMEOUT and the launch goes on
-// without waiting: no CTA leaves while another may still push to it.
+// A wait that runs out (wait_polls) records AMCFD_E_TIMEOUT, which fails the step, and goes
+// on for kChainGrace: every phase is armed once, when the one before it is over, and takes
+// exactly its own visit's transactions, so a launch whose budget ran out ends like any
+// other and nothing is under way to a CTA that leaves.  Should the values not come
+// then either, the warp leaves its visits out from there on (it neither arms nor pushes),
+// and waits that long once more before the last cluster barrier.
 //
 // A box that has outgrown the lines' shared memory since the launch was chosen
 // (kChainLines lines a CTA, kChainCells cells a line) is solved in place in
@@ -1793,21 +1797,43 @@ __device__ __forceinline__ void st_async(unsigned addr, unsigned bar, double v)
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr),
                  "l"(__double_as_longlong(v)), "r"(bar) : "memory");
 }
-// Bounded wait of the whole warp on phase `parity`, with cluster-scope acquire.
+__device__ __forceinline__ unsigned long long global_ns()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+constexpr unsigned long long kChainGrace = 500000000ull;  // ns
+constexpr int kTryPolls = 64;  // a try_wait that finds nothing returns after 4 us, 64 polls' time
+// Bounded wait of the whole warp on phase `parity`, with cluster-scope acquire.  Past
+// `polls` it records AMCFD_E_TIMEOUT and goes on for kChainGrace, whoever else has recorded
+// an error: the values are on their way, and a phase must not be left open while others
+// push to it.  False when they did not come in that time either.  (A budget below one
+// try_wait is counted in test_waits, 40 ns each.)
 __device__ __forceinline__ bool chain_wait(unsigned bar, unsigned parity, Status *st, long long polls)
 {
-    for (long long it = 0;; ++it) {
+    const bool brief = polls < kTryPolls;
+    unsigned long long until = 0;
+    for (long long it = 0;; it += brief ? 1 : kTryPolls) {
         unsigned done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-            " selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+        if (brief)
+            asm volatile(
+                "{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+                " selp.u32 %0, 1, 0, p;\n}\n"
+                : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+        else
+            asm volatile(
+                "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+                " selp.u32 %0, 1, 0, p;\n}\n"
+                : "=r"(done) : "r"(bar), "r"(parity) : "memory");
         if (__all_sync(0xffffffffu, done)) return true;
-        if ((it & 63) == 63 && __any_sync(0xffffffffu, *(volatile int *)&st->error != 0)) return false;
-        if (it > polls) {
+        if (it <= polls) continue;
+        const unsigned long long now = global_ns();
+        if (until == 0) {
             if ((threadIdx.x & 31) == 0 && atomicCAS(&st->error, 0, AMCFD_E_TIMEOUT) == 0) st->error_where = -6;
-            return false;
+            until = now + kChainGrace;
         }
+        if (__any_sync(0xffffffffu, now > until)) return false;
     }
 }
 
@@ -2230,18 +2256,20 @@ mom_chain_kernel(Params p, Fields<T> g, double *red, int nb_region, double *rcel
                 ChainLine<T> &ln = lines[l];
                 const int c = (f.j + f.k) & 1;
                 const int need = chain_waits<EXACT>(vs, c, f.in), to = chain_pushes<EXACT>(vs, c, f.in);
-                if (need) {
+                if (need && ok) {
                     if (lane == 0)
                         mbar_expect_tx(reinterpret_cast<uint64_t *>(&info[l].bar), (unsigned)(__popc(need) * n * sizeof(T)));
                     __syncwarp();
-                    if (ok) ok = chain_wait(smem_u32(&f.bar), par >> s & 1, st, p.wait_polls);
+                    ok = chain_wait(smem_u32(&f.bar), par >> s & 1, st, p.wait_polls);
                     par ^= 1u << s;
                 }
                 T *out = vs == 3 ? phi + cidx(i0, f.j, f.k, nj, nip) : nullptr;
-                if (n <= 32)
-                    chain_visit<T, 1>(ln, f, n, to, out);
-                else
-                    chain_visit<T, 2>(ln, f, n, to, out);
+                if (ok) {
+                    if (n <= 32)
+                        chain_visit<T, 1>(ln, f, n, to, out);
+                    else
+                        chain_visit<T, 2>(ln, f, n, to, out);
+                }
                 __syncwarp();
                 if (s) {
                     ++v[1];
@@ -2278,6 +2306,10 @@ mom_chain_kernel(Params p, Fields<T> g, double *red, int nb_region, double *rcel
         if (idle == 0) beside(ivar, t, nt);
         cluster_barrier();
     }
+    // after a wait that gave up for good: what was pushed to this CTA since lands before it leaves
+    if (!ok)
+        for (const unsigned long long until = global_ns() + kChainGrace; global_ns() < until;) __nanosleep(1000);
+    __syncwarp();
     for (int q = t; q < b.n; q += nt) {
         int i, j, k;
         box_cell(b, q, i, j, k);
