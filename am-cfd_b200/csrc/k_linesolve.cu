@@ -219,7 +219,12 @@ __global__ void sweep_exact_kernel(Params p, Fields<T> g, T *phi, int *flags, co
 //     plane k + 1 and 2 ks of plane k - 1; version 0 is the unknown before the solve,
 //     which its line keeps in phi until its last visit.  A line goes on to its next
 //     visit only after these readers' own visits, so no version passes unseen.  The
-//     words of line j + 1 are loaded while line j is solved, and again if too early;
+//     words of line j + 1 are loaded while line j is solved, and again if too early.
+//     Relaxed accesses of different words order nothing, so a word's versions, stored by
+//     different CTAs, are put in order by the word itself: the lane that stores version
+//     v + 1 has loaded the same word and found version v in it (at line j - 1 as a word
+//     of the north line; of a row's first line, separately), and a store that follows
+//     a load of its word comes after the store that the load saw;
 //   * a second warp brings the coefficient rows of the next lines by bulk copies.
 // Rows are handed out by an atomic ticket in the order (ks, k, s), which every
 // dependency precedes: the smallest outstanding row is always runnable, so no
@@ -256,14 +261,6 @@ template <> struct RowWord<double> {
     }
     __device__ __forceinline__ double value() const { return __hiloint2double((int)(unsigned)b, (int)(unsigned)a); }
 };
-template <typename T>
-__device__ __forceinline__ bool row_load(const unsigned long long *xc, size_t c, unsigned tag, T &v)
-{
-    RowWord<T> w;
-    w.load(xc, c);
-    v = w.value();
-    return w.holds(tag);
-}
 __device__ __forceinline__ void row_store(unsigned long long *xc, size_t c, unsigned tag, float v)
 {
     const unsigned long long w = ((unsigned long long)tag << 32) | __float_as_uint(v);
@@ -421,18 +418,6 @@ __global__ void __launch_bounds__(64) sweep_rows_kernel(Params p, Fields<T> g, T
 #pragma unroll 1
             for (int j = j0; j <= j1; ++j, row += sj) {
                 it = 0;
-                // a plane of one line: its visits depend on nothing of one another, but their
-                // versions must land in turn
-                if (j0 == j1 && v > 0)
-                    for (;;) {
-                        bool turn = true;
-#pragma unroll
-                        for (int c = 0; c < L; ++c) {
-                            T y;
-                            turn = turn && (a + c >= n || row_load(xc, row + a + c, tag0 + (unsigned)v, y));
-                        }
-                        if (__all_sync(full, turn) || !(ok = again(k * nj + j))) break;
-                    }
                 while (ok && !arrived(cur, j < j1)) {
                     reload(cur, row, j < j1);
                     ok = again(k * nj + j);
@@ -450,10 +435,26 @@ __global__ void __launch_bounds__(64) sweep_rows_kernel(Params p, Fields<T> g, T
                     cf[c] = sl[S_CF * nmax + w];
                     pr[c] = sl[S_PR * nmax + w];
                 }
+                // a row's first line: its own words, to be seen at version v before they are
+                // stored to (a later line's are, as the north words of the line before it)
+                RowWord<T> own[L];
+                if (j == j0 && v > 0)
+#pragma unroll
+                    for (int c = 0; c < L; ++c) own[c].load(xc, row + at[c]);
                 // the next line's neighbours start while this line is solved
                 if (j < j1) issue(nxt, row + sj, j + 1 < j1);
                 scan_line_lanes<T, L>(n, e, cf, pr, cur.lo, cur.hi);
                 if (j < j1) reload(nxt, row + sj, j + 1 < j1);
+                if (j == j0 && v > 0)
+                    while (ok) {
+                        bool turn = true;
+#pragma unroll
+                        for (int c = 0; c < L; ++c) turn = turn && (a + c >= n || own[c].holds(tag0 + (unsigned)v));
+                        if (__all_sync(full, turn)) break;
+#pragma unroll
+                        for (int c = 0; c < L; ++c) own[c].load(xc, row + at[c]);
+                        ok = again(k * nj + j);
+                    }
 #pragma unroll
                 for (int c = 0; c < L; ++c) {
                     x[c] = e[c];
