@@ -31,7 +31,7 @@ extern "C" int amcfd_run_batch(amcfd_ctx *const *ctxs, int n, int nsteps, int nt
     std::vector<amcfd_step_report> rep(n);
     // The first step of the first context of each kind runs here, alone: it loads
     // every kernel that kind launches (a kernel's first launch loads its module,
-    // which must not happen while another thread captures a graph).  A kind that a
+    // which must not happen while another thread captures a graph).  A kind of which a
     // context here has stepped before is loaded already (its first context's step
     // alone took 5.6 of 35 ms on eight instances of up to 240x120x60 cells, two steps).
     std::vector<int> kinds;

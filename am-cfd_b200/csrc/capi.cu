@@ -144,6 +144,7 @@ struct amcfd_ctx {
     void *ws_save[4] = {};         // h, p, T, f_l at the start of the step
     long long ws_accepted = 0, ws_rejected = 0;
     int ws_fallback = 0;           // the last step's prediction was rejected
+    int stepped_kind = -1;         // ctx_kind at the end of the last step (-1: none yet)
 };
 
 #define CK(call)                                                                          \
@@ -154,6 +155,10 @@ struct amcfd_ctx {
             return AMCFD_E_CUDA;                                                          \
         }                                                                                 \
     } while (0)
+
+namespace amcfd {
+int ctx_kind(const amcfd_ctx *ctx);
+}
 
 static int fail(amcfd_ctx *ctx, int code, const std::string &msg)
 {
@@ -1573,6 +1578,7 @@ int amcfd_step(amcfd_ctx *ctx, amcfd_step_report *report)
     }
     CK(cudaStreamSynchronize(ctx->stream));
     CK(cudaGetLastError());
+    ctx->stepped_kind = amcfd::ctx_kind(ctx);
     fill_report(ctx, report);
     return 0;
 }
@@ -1585,13 +1591,38 @@ static int field_ptr(amcfd_ctx *ctx, const char *name, void **ptr);
 }
 namespace amcfd {
 void ctx_report(amcfd_ctx *ctx, amcfd_step_report *r) { fill_report(ctx, r); }
-// The kernel set a context launches: its precision, defect correction, order and
-// graph use (contexts of one kind load the same kernels).
+// The kernels a context's steps launch, as a key: every option and feature by which the
+// host chooses between kernels.  (The instantiations that follow from the grid's size
+// are loaded at creation, which sets their attributes.)
 int ctx_kind(const amcfd_ctx *ctx)
 {
-    return ctx->precision + 2 * (ctx->dc ? 1 : 0) + 4 * ctx->order + 8 * (ctx->use_graphs ? 1 : 0);
+    const amcfd_params &q = ctx->prm;
+    int key = 0;
+    auto put = [&](int v, int bits) { key = key << bits | v; };
+    put(ctx->precision == AMCFD_PREC_FP64, 1);
+    put(ctx->dc, 1);
+    put(ctx->order, 1);
+    put(ctx->use_graphs, 1);
+    put(ctx->host_loop || q.maxit > kMaxChain, 1);
+    put(ctx->events, 1);
+    put(ctx->serial_launch, 1);
+    put(ctx->pass_launch, 1);
+    put(ctx->small_mode + 1, 2);
+    put(ctx->mom_cluster > 1, 1);
+    put((ctx->precision == AMCFD_PREC_FP64 ? ctx->I64.box_grid : ctx->I32.box_grid) > 0, 1);
+    put((ctx->precision == AMCFD_PREC_FP64 ? ctx->I64.chain_nc : ctx->I32.chain_nc) > 0, 1);
+    put(q.scheme & 3, 2);
+    put(q.species != 0, 1);
+    put(q.powderbed != 0, 1);
+    put(q.movingmesh != 0, 1);
+    put(q.solidification != 0, 1);
+    put(q.freesurface != 0, 1);
+    put(q.steady != 0, 1);
+    put(ctx->ws_mode, 2);
+    return key;
 }
-bool ctx_stepped(const amcfd_ctx *ctx) { return ctx->itertot > 0; }
+// Whether the context has run a step of the kind it is now.
+bool ctx_stepped(const amcfd_ctx *ctx) { return ctx->stepped_kind == ctx_kind(ctx); }
 double ctx_delt(const amcfd_ctx *ctx) { return ctx->delt; }
 double ctx_outtime(const amcfd_ctx *ctx) { return ctx->outtime; }
 const amcfd_params &ctx_params(const amcfd_ctx *ctx) { return ctx->prm; }
