@@ -1265,7 +1265,9 @@ static void ws_after(amcfd_ctx *ctx, Inst<T> &I)
 // with CUDA events on the context stream (one untimed round, then the minimum of
 // three rounds in rotated order) on this grid; the fastest of each is kept unless
 // the options pin it.  The assembly runs in place (everything it writes is formed
-// again by the first outer iteration); the sweep passes run on a scratch field.
+// again by the first outer iteration); the sweep passes run on a scratch field.  The
+// stride is that of the pipelined launch, which is timed also where the domain is small
+// enough for every line to have its own warp: a powder bed may grow out of that.
 template <typename T>
 static int autotune(amcfd_ctx *ctx, Inst<T> &I)
 {
@@ -1276,6 +1278,8 @@ static int autotune(amcfd_ctx *ctx, Inst<T> &I)
     bool pipe = I.pipe_grid > 0;
     if constexpr (sizeof(T) == sizeof(double))
         if (I.dc_on) pipe = I.pipe_grid_dc > 0;
+    const bool resident = I.resident;
+    I.resident = false;
     float best_asm[3], best_sw[3];
     for (int c = 0; c < 3; ++c) best_asm[c] = best_sw[c] = INFINITY;
     auto set_seg = [&](int seg) {
@@ -1340,6 +1344,7 @@ static int autotune(amcfd_ctx *ctx, Inst<T> &I)
         }
         for (int q = 0; q < 3; ++q) ctx->tune_ms[3 + q] = best_sw[q];
     }
+    I.resident = resident;
     ctx->launches += 4 * 3 * 3;
     return 0;
 }

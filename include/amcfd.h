@@ -300,7 +300,8 @@ long long amcfd_kernel_launches(const amcfd_ctx *ctx);
 int amcfd_tuning(const amcfd_ctx *ctx, int *asm_kseg, int *sweep_warps, double *times);
 /* The planes between successive passes in the work order of the pipelined red-black
  * line solve (autotuned among 8, 16, 32; default 16), or 0 when the passes take a
- * launch each.  No counterpart in the reference (its sweeps are sequential loops). */
+ * launch each.  A domain small enough for every line to have its own warp does not use it
+ * until it grows (powder bed).  No counterpart in the reference (its sweeps are sequential loops). */
 int amcfd_pipe_stride(const amcfd_ctx *ctx, int *stride);
 
 /* Parameter sweep over independent instances: runs nsteps time steps of every
