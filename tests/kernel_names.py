@@ -1,5 +1,6 @@
 """Names of the kernels that a stretch of code launches, for tests of which launch a call
-takes."""
+takes.  Of direct launches only: for a replayed graph the profiler can report the names of
+one that has been destroyed."""
 import re
 from collections import Counter
 
