@@ -1213,7 +1213,7 @@ static int ws_residual(amcfd_ctx *ctx, Inst<T> &I, double &r)
         CK(cudaStreamSynchronize(ctx->stream));
         r = INFINITY;
     }
-    ctx->launches += 3;
+    ctx->launches += 2;
     return 0;
 }
 
