@@ -1,10 +1,7 @@
-"""Which form of the energy assembly a scheme takes, and the exponential scheme's launch
-shapes against one another: its A(0) is 0 / 0, so it has no short form of a cell without
-flow, and the launch shapes made for that form are not for it."""
+"""The exponential scheme's launch shapes of the energy assembly against one another (which
+form it takes: test_launch_names.py)."""
 import numpy as np
 import pytest
-
-from kernel_names import launched
 
 pytestmark = pytest.mark.gpu
 
@@ -20,20 +17,6 @@ def _deck(tmp, scheme, nx, ny, nz):
                z_zones=[(15e-6 * nz, nz, 1.0)], power=250.0, scheme=scheme,
                single_track=(1.0, 33e-6 * nx * 0.4, 33e-6 * ny * 0.5, 1.0), finaltime=1e-3)
     return amcfd.Deck(d.write(str(tmp / scheme)))
-
-
-# at most one CTA a SM, at most three, more
-@pytest.mark.parametrize("nx,ny,nz", [(60, 30, 20), (120, 60, 40), (200, 100, 60)])
-@pytest.mark.parametrize("prec,t,dc,occ", [(0, "double", "false", 2), (1, "float", "false", 3), (2, "double", "true", 2)])
-def test_exponential_scheme_takes_the_long_form(prec, t, dc, occ, nx, ny, nz, tmp_path):
-    import amcfd
-    deck = _deck(tmp_path, "exponential_law", nx, ny, nz)
-    s = amcfd.Solver(deck, order=amcfd.ORDER_REDBLACK, precision=prec, check_finite=0)
-    s.run_phase("laser")
-    n = launched(lambda: s.run_phase("energy_assemble"))
-    forms = [k.replace(" ", "") for k in n if k.startswith("energy_assemble_kernel")]
-    assert forms == [f"energy_assemble_kernel<{t},2,{dc},false,{occ}>"], n
-    s.close()
 
 
 @pytest.mark.parametrize("prec", [0, 1])  # (defect correction keeps its coefficients to itself)
