@@ -672,10 +672,10 @@ static void swap_props(Inst<T> &I)
 // iteration, fit the cluster's shared memory; when pinned, the one-CTA chain, for
 // red-black runs whose box fits one CTA's.  Both stay correct, only slower, if the
 // box has grown past that since.  Where there is no cluster launch the automatic
-// mode takes the one-CTA chain only without the cooperative box solve: on the 400x200x100 deck the cooperative path took 0.099
-// against 0.139 ms an outer iteration for boxes of 1300-2200 cells and 0.100
-// against 0.176 for 2600-3100 cells; on the 120x60x40 deck 0.093 against 0.101
-// (1400-1600 cells) and the same 0.090 for 800-1000 cells.
+// mode takes the one-CTA chain only without the cooperative box solve: on the
+// 400x200x100 deck the cooperative path took 0.099 against 0.139 ms an outer iteration
+// for boxes of 1300-2200 cells and 0.100 against 0.176 for 2600-3100 cells; on the
+// 120x60x40 deck 0.093 against 0.101 (1400-1600 cells) and the same 0.090 for 800-1000.
 template <typename T>
 static bool small_allowed(const amcfd_ctx *ctx, const Inst<T> &I)
 {

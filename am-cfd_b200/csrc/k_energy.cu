@@ -493,9 +493,9 @@ __device__ void reset_scan_candidates(const Params &p, Fields<T> &g)
 
 // ---------------------------------------------------------------------------
 // getMeltPoolShape (BoundCondManager.cpp:280-447), one CTA.  The scans along
-// i/j/k are evaluated per column in parallel; the folds whose result depends on
-// order (the NaN behaviour of std::max/min) run sequentially in thread 0.
-// Also activates the momentum box and builds its exact-order ticket list.
+// i/j/k are evaluated per column in parallel, and so are the folds whose result
+// depends on order (the NaN behaviour of std::max/min).  Also activates the momentum
+// box (its exact-order ticket list is box_tickets_kernel's).
 // ---------------------------------------------------------------------------
 // The reference's folds acc = f(x_i, acc) in ascending i over the flagged columns,
 // with f = std::max or std::min as the reference folds (maxd/mind): a NaN element

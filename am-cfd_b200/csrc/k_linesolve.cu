@@ -231,7 +231,8 @@ __global__ void sweep_exact_kernel(Params p, Fields<T> g, T *phi, int *flags, co
 // co-residency is assumed.  Waits are bounded (wait_polls).
 // The line arithmetic is solve_staged's and scan_line's: the same bits.
 // Measured (us a solve, FP64): 61x31x21 cells 635 -> 282, 120x60x40 1352 -> 879, 40x200x30
-// 1554 -> 577; FP32 100x48x30 957 -> 414.  A row lags the one before by one to two visits of
+// 1554 -> 577; FP32 100x48x30 957 -> 414 (2-4 us more since, for the look at a first line's
+// own words).  A row lags the one before by one to two visits of
 // 1.3 us (scans 0.5, a word's way between SMs 0.3-0.5, the rest loads and stores).
 // ---------------------------------------------------------------------------
 template <typename T> constexpr int kRowW = (int)sizeof(T) / 4;  // exchange words a cell
@@ -666,7 +667,7 @@ __device__ __forceinline__ void factor_round(T (&wc)[16 / sizeof(T)], T (&wi)[16
 }
 
 // One pass over the interior x-line (j, k) by the calling warp; sq/spr are the
-// warp's qr/pr buffers (2 R RC elements).  The same operations whichever kernel
+// warp's qr/pr buffers (nip elements each).  The same operations whichever kernel
 // calls it, so the per-pass launches and the pipelined launch give the same bits.
 template <typename T>
 __device__ __forceinline__ void pf_l1(const T *ptr)
@@ -1708,8 +1709,8 @@ template <typename T> void set_sweep_smem_limit(size_t smem)
 // Exact-order sweep by rows: the exchange words it needs (0 for lines past 128 cells, where
 // one warp a row fell behind the visits dealt out singly: 1960 against 1930 us a solve on
 // 160x80x50 cells, 4740 against 3460 on 300x150x60), with its shared-memory limit raised; `grid` receives its
-// (one-warp) CTAs: the rows a wave touches, 2 in 3 of a plane's lines, and a few that
-// wait, at most the rows there are and what is resident at once.
+// CTAs, one solving warp each: the rows a wave touches, 2 in 3 of a plane's lines, and a few
+// that wait, at most the rows there are and what is resident at once.
 template <typename T> size_t setup_rows(const Params &p, int sm_count, int &grid)
 {
     const size_t need = rows_smem<T>(p);

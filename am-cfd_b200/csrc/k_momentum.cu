@@ -1723,15 +1723,15 @@ mom_cluster_post_kernel(Params p, Fields<T> g, T *scratch, int smem_elems, const
 //     live, by st.async: the stores complete on the receiving line's mbarrier, so
 //     a value and the news of it travel together in one hop;
 //   * launches become cluster barriers, about 1 us each with the stores before
-//     them (14 of them), and the boundary values of the next equation, the part of
-//     its coefficients that does not depend on the flow, and the residual sums run
-//     on the warps without a line while the others solve.
+//     them (11 of them: after cleanVelocities, the first boundary values and the
+//     velocity correction, and two an equation), and the boundary values of the next
+//     equation, the part of its coefficients that does not depend on the flow, and the
+//     residual sums run on the warps without a line while the others solve.
 // Measured (120x60x40 deck, box of 1600 cells, 98 lines on 16 CTAs): 47 us a chain in FP32
 // and 79 in FP64, of which the eight passes take 4.2-5.6 us an equation and the assembly
 // 3-5 (FP32) and 7-10 (FP64), a serial stretch of divisions; the chain in one piece of
-// assembly 52 and 90; the step (with fields read) 4.78 ms in FP32 and 6.92 in FP64 with the
-// multi-launch chain, 4.15 and 5.78 with this one, the reference's order on 61x31x21
-// cells 31.8 and 18.1 ms.  L2 prefetches of the rows the first assembly reads gained
+// assembly 52 and 90; the multi-launch chain 94 and 150, in the reference's order on 61x31x21
+// cells 847 against 155.  L2 prefetches of the rows the first assembly reads gained
 // nothing (66.5 -> 68 us on the 400x200x100 deck).
 // The arithmetic is that of the multi-launch chain operation for operation
 // (line_rhs, the scans of solve_line_regs, factor_cell; the residual sums are

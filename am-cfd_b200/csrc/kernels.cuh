@@ -103,7 +103,7 @@ struct Inst {
     int grid_1d = 0;          // grid of the pointwise kernels
     int exact_grid = 0;       // CTAs of the persistent exact-order line sweep
     // the exact-order sweep of the whole domain by rows: exchange words (null: by single
-    // visits) and CTAs of one warp
+    // visits) and CTAs (a solving warp and one that brings its coefficient rows)
     unsigned long long *xrow = nullptr;
     int row_grid = 0;
     int exact_warps = 4;      // warps per CTA in the line sweeps

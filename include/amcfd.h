@@ -162,7 +162,9 @@ typedef struct amcfd_options {
     int wait_polls;      /* polls (about 64 ns each) a warp of a line sweep (the exact-order
                             sweep, the red-black passes of a solve in one launch, the
                             momentum launches) waits for a neighbouring line before the step fails with
-                            AMCFD_E_TIMEOUT; 0 = the default 2^24 (about one second).  The
+                            AMCFD_E_TIMEOUT; 0 = the default 2^24 (about one second).  (A
+                            momentum chain in one launch records the error and still runs
+                            to its end, a few seconds later at most.)  The
                             reference has no such wait (its sweeps are sequential). */
     int autotune;        /* 1: at creation, time the candidate launch shapes of the energy
                             assembly (planes per CTA) and of the red-black line sweeps (lines
